@@ -174,7 +174,8 @@ __global__ void k_generator_mul(uint64_t *__restrict__ out, const uint4 *__restr
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
   using T = typename F::T;
-  gm::xyzz_t<F> acc;
+  using FA = typename gm::OutOfLine<F>::type;
+  gm::xyzz_t<FA> acc;
   gm::xyzz_set_inf(acc);
   for (int l = 0; l < limbs; l++) {
     uint64_t k = scalars[i * limbs + l];
@@ -183,7 +184,7 @@ __global__ void k_generator_mul(uint64_t *__restrict__ out, const uint4 *__restr
       k &= k - 1;
       T x, y;
       gm::load_base<F>(x, y, table + (size_t)(64 * l + b) * gm::Rec<F>::U4);
-      gm::xyzz_madd<F>(acc, x, y);
+      gm::xyzz_madd<FA>(acc, x, y);
     }
   }
   constexpr int Hw = F::LIMBS / 2;
@@ -193,9 +194,9 @@ __global__ void k_generator_mul(uint64_t *__restrict__ out, const uint4 *__restr
     dst[2 * Hw] = 1;  // infinity flag byte, pad bytes zero
     return;
   }
-  const T I = F::inv(F::mul(acc.ZZ, acc.ZZZ));
-  T x = F::mul(acc.X, F::mul(I, acc.ZZZ));
-  T y = F::mul(acc.Y, F::mul(I, acc.ZZ));
+  const T I = FA::inv(FA::mul(acc.ZZ, acc.ZZZ));
+  T x = FA::mul(acc.X, FA::mul(I, acc.ZZZ));
+  T y = FA::mul(acc.Y, FA::mul(I, acc.ZZ));
   gm::store_ref<F>(dst, x);
   gm::store_ref<F>(dst + Hw, y);
   dst[2 * Hw] = 0;
@@ -224,19 +225,20 @@ template <class F>
 __global__ void k_proj_sum(uint64_t *__restrict__ out, const uint64_t *__restrict__ in, int n) {
   if (blockIdx.x != 0 || threadIdx.x != 0) return;
   constexpr int Hw = F::LIMBS / 2;
-  gm::xyzz_t<F> acc;
+  using FA = typename gm::OutOfLine<F>::type;
+  gm::xyzz_t<FA> acc;
   gm::xyzz_set_inf(acc);
   for (int i = 0; i < n; i++) {
     typename F::T X, Y, Z;
     gm::load_ref<F>(X, in + (size_t)i * 3 * Hw);
     gm::load_ref<F>(Y, in + (size_t)i * 3 * Hw + Hw);
     gm::load_ref<F>(Z, in + (size_t)i * 3 * Hw + 2 * Hw);
-    gm::xyzz_t<F> p;
-    gm::proj_to_xyzz<F>(p, X, Y, Z);
-    gm::xyzz_add_cold<F>(acc, p);
+    gm::xyzz_t<FA> p;
+    gm::proj_to_xyzz<FA>(p, X, Y, Z);
+    gm::xyzz_add_cold<FA>(acc, p);
   }
   typename F::T X, Y, Z;
-  gm::xyzz_to_proj<F>(X, Y, Z, acc);
+  gm::xyzz_to_proj<FA>(X, Y, Z, acc);
   gm::store_ref<F>(out, X);
   gm::store_ref<F>(out + Hw, Y);
   gm::store_ref<F>(out + 2 * Hw, Z);

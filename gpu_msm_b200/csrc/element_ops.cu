@@ -24,18 +24,19 @@
 //     (src/curve.cu:72-227), so inputs that share x but are not P and -P
 //     give its result too;
 //   - scalar multiplication runs MSB-first double-and-add in XYZZ
-//     coordinates on one quad (xyzz_quad.cuh) and inverts once at the end:
+//     coordinates on one warp (xyzz_warp.cuh) and inverts once at the end:
 //     one inversion instead of one per doubling and addition.  For points
 //     on the curve the group law makes its result equal to the reference's
 //     affine double-and-add (src/curve.cu:230-268).
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "../../include/gpu_msm_b200.h"
 #include "msm_engine.h"
 #include "msm_kernels.cuh"
-#include "xyzz_quad.cuh"
+#include "xyzz_warp.cuh"
 
 namespace {
 
@@ -341,36 +342,41 @@ __global__ void k_point_elem(int op, uint64_t *r, const uint64_t *p, const uint6
   out.store(r);
 }
 
-// k * P, one warp: each quad runs the same double-and-add over the scalar
-// bits (MSB first) with the quad-parallel XYZZ formulas; lane 0 stores.
-// `scalar` holds `limbs` u64 limbs; when it is null the scalar is k64.
+template <class F>
+struct FieldOf {
+  using type = typename std::conditional<sizeof(typename F::T) == sizeof(fp_t), gm::Fp, gm::Fp2>::type;
+};
+
+// k * P, one warp: double-and-add over the scalar bits (MSB first) with the
+// warp-parallel XYZZ formulas; lane 0 stores.  `scalar` holds `limbs` u64
+// limbs; when it is null the scalar is k64.
 template <class F>
 __global__ void k_point_smul(uint64_t *r, const uint64_t *p, const uint64_t *scalar, int limbs, uint64_t k64) {
   using T = typename F::T;
+  using G = typename FieldOf<F>::type;
+  using W = gm::WF<G>;
+  gm::w_setup();
   RefPt<F> a;
   a.load(p);
-  gm::xyzz_t<F> acc;
-  gm::xyzz_set_inf(acc);
+  gm::wpt<G> acc = gm::w_inf<G>();
   if (!a.inf) {
-    gm::xyzz_t<F> base;
-    base.X = a.x;
-    base.Y = a.y;
-    base.ZZ = F::one();
-    base.ZZZ = F::one();
+    const uint32_t *w32 = reinterpret_cast<const uint32_t *>(p);
+    const typename W::E x = W::load_words(w32), y = W::load_words(w32 + W::WORDS);
     const int nl = scalar ? limbs : 1;
     for (int l = nl - 1; l >= 0; l--) {
       const uint64_t w = scalar ? scalar[l] : k64;
       for (int bit = 63; bit >= 0; bit--) {
-        gm::q_dbl<F>(acc);
-        if ((w >> bit) & 1u) gm::q_add<F>(acc, base);
+        acc = gm::w_dbl<G>(acc);
+        if ((w >> bit) & 1u) acc = gm::w_madd<G>(acc, x, y);
       }
     }
   }
   RefPt<F> out = RefPt<F>::infinity();
-  if (!gm::xyzz_is_inf(acc)) {
+  if (!acc.inf) {
     // x = X / ZZ = X ZZZ I, y = Y / ZZZ = Y ZZ I with I = 1 / (ZZ ZZZ)
-    const T I = F::inv(F::mul(acc.ZZ, acc.ZZZ));
-    out = RefPt<F>{F::mul(acc.X, F::mul(I, acc.ZZZ)), F::mul(acc.Y, F::mul(I, acc.ZZ)), false};
+    const T ZZ = W::canon(acc.ZZ), ZZZ = W::canon(acc.ZZZ);
+    const T I = F::inv(F::mul(ZZ, ZZZ));
+    out = RefPt<F>{F::mul(W::canon(acc.X), F::mul(I, ZZZ)), F::mul(W::canon(acc.Y), F::mul(I, ZZ)), false};
   }
   if (threadIdx.x == 0) out.store(r);
 }
@@ -477,7 +483,7 @@ int point_elem(gm_stream_t stream, uint32_t gpu_index, int op, void *d_r, const 
   if (op == GM_PT_SCALAR_MUL || op == GM_PT_SCALAR_MUL_U64) {
     // a scalar of no limbs is zero (src/curve.cu:240-249): pass one zero word
     const bool limbs_given = op == GM_PT_SCALAR_MUL && scalar_limbs > 0;
-    k_point_smul<F><<<1, 32, 0, s>>>((uint64_t *)d_r, (const uint64_t *)d_p, limbs_given ? d_scalar : nullptr,
+    k_point_smul<F><<<1, 32, gm::w_smem_bytes<typename FieldOf<F>::type>(1), s>>>((uint64_t *)d_r, (const uint64_t *)d_p, limbs_given ? d_scalar : nullptr,
                                      limbs_given ? scalar_limbs : 1,
                                      op == GM_PT_SCALAR_MUL_U64 ? scalar_u64 : 0ull);
     return launched("k_point_smul");

@@ -88,8 +88,7 @@ void batch_class_layout(BatchClassPlan &cp, int limbs, int sms, int dev) {
   cp.o_tail = cv.take<xyzz_t<F>>(cp.nthreads);
   cp.o_hk = cv.take<int32_t>(cp.nthreads);
   cp.o_tk = cv.take<int32_t>(cp.nthreads);
-  cp.rl.plan<F>(groups, cp.dp.B, (int64_t)sms * level0_blocks_per_sm<F>(dev) * 128, cv, coop_wave_threads<F>(dev, sms));
-  cp.rl.sms = sms;
+  cp.rl.plan<F>(groups, cp.dp.B, (int64_t)sms * level0_blocks_per_sm<F>(dev) * 128, sms, cv);
   cp.rl.dev = dev;
   cp.long_cap = cp.nthreads / FIX_SHORT + 1;
   cp.o_longq = cv.take<int32_t>((size_t)(1 + cp.long_cap));
@@ -149,9 +148,9 @@ int batch_class_finish(const BatchClassPlan &cp, cudaStream_t s, uint64_t *resul
   rc = reduce_launch<F>(s, cp.rl, cb.buckets, cb.offsets, cp.ws, &src, launches);
   if (rc) return rc;
   // precomputed mode: one window per MSM, so the combination is a conversion
-  k_combine_quad<F><<<grid_for((int64_t)Coop<F>::LANES * cp.count, 128), 128, 0, s>>>(
-      src, cp.count, cp.pc_stride ? 1 : cp.dp.W, cp.c, cb.out_index, results);
-  GM_CHECK_LAUNCH("k_combine_quad");
+  k_combine<F><<<(unsigned)cp.count, 32 * COMBINE_WARPS, w_sum_smem<F>(COMBINE_WARPS), s>>>(
+      src, cp.pc_stride ? 1 : cp.dp.W, cp.c, cb.out_index, results);
+  GM_CHECK_LAUNCH("k_combine");
   (*launches)++;
   return GM_OK;
 }

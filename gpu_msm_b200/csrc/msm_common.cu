@@ -21,7 +21,6 @@
 #include <vector>
 
 #include "../../include/gpu_msm_b200.h"
-#include "host_arith.h"
 #include "msm_engine.h"
 
 namespace gm {
@@ -149,9 +148,8 @@ int64_t launches_and_reset() {
 }
 
 // ---------------------------------------------------------------------------
-// host tail: pinned slots and stream-ordered host functions
+// pinned host slots (descriptors, window sums and results on their way)
 // ---------------------------------------------------------------------------
-constexpr size_t TAIL_SLOT_BYTES = PINNED_SLOT_BYTES;  // >= 257 windows x 448 B + 336 B
 static std::mutex g_pin_mu;
 static std::vector<void *> g_pin_free;
 // Slots whose last copy is still pending: returned to the free list once
@@ -164,10 +162,6 @@ struct PendingSlot {
 };
 static std::vector<PendingSlot> g_pin_pending;
 static std::map<int, std::vector<cudaEvent_t>> g_free_events;  // per device
-static bool g_host_tail = true;
-
-bool host_tail_enabled() { return g_host_tail; }
-void set_host_tail_enabled(bool on) { g_host_tail = on; }
 
 // caller holds g_pin_mu
 static void reclaim_completed_slots() {
@@ -228,56 +222,6 @@ int enqueue_pinned_release(cudaStream_t s, void *slot) {
   std::lock_guard<std::mutex> lk(g_pin_mu);
   g_pin_pending.push_back(PendingSlot{slot, ev, dev});
   return GM_OK;
-}
-
-struct TailCtx {
-  int group, W, c;
-  char *slot;
-};
-
-// Horner over the window sums in the slot; the result goes after them.
-static void CUDART_CB tail_compute(void *p) {
-  auto *t = static_cast<TailCtx *>(p);
-  if (t->group == 1) {
-    uint64_t *out = reinterpret_cast<uint64_t *>(t->slot + (size_t)t->W * sizeof(gm_host::HXyzz<gm_host::F1>));
-    gm_host::horner_to_proj<gm_host::F1>(out, reinterpret_cast<const gm_host::HXyzz<gm_host::F1> *>(t->slot), t->W,
-                                         t->c);
-  } else {
-    uint64_t *out = reinterpret_cast<uint64_t *>(t->slot + (size_t)t->W * sizeof(gm_host::HXyzz<gm_host::F2>));
-    gm_host::horner_to_proj<gm_host::F2>(out, reinterpret_cast<const gm_host::HXyzz<gm_host::F2> *>(t->slot), t->W,
-                                         t->c);
-  }
-  delete t;
-}
-
-int enqueue_host_tail(cudaStream_t s, int group, const void *d_sums, int W, int c, uint64_t *d_out) {
-  const size_t elem = group == 1 ? sizeof(gm_host::HXyzz<gm_host::F1>) : sizeof(gm_host::HXyzz<gm_host::F2>);
-  const size_t out_bytes = 3 * (group == 1 ? 7 : 14) * sizeof(uint64_t);
-  if ((size_t)W * elem + out_bytes > TAIL_SLOT_BYTES) {
-    set_last_error("too many windows for the host tail slot");
-    return GM_ERR_ARG;
-  }
-  void *slot = nullptr;
-  int rc = pinned_acquire(&slot);
-  if (rc) return rc;
-  auto *t = new TailCtx{group, W, c, static_cast<char *>(slot)};
-  cudaError_t e = cudaMemcpyAsync(slot, d_sums, (size_t)W * elem, cudaMemcpyDeviceToHost, s);
-  if (e != cudaSuccess) {
-    pinned_release(slot);
-    delete t;
-    return record_error(e, "tail D2H");
-  }
-  e = cudaLaunchHostFunc(s, tail_compute, t);
-  if (e != cudaSuccess) {
-    delete t;
-    // the D2H may still write the slot: release it in stream order
-    enqueue_pinned_release(s, slot);
-    return record_error(e, "tail host function");
-  }
-  e = cudaMemcpyAsync(d_out, static_cast<char *>(slot) + (size_t)W * elem, out_bytes, cudaMemcpyHostToDevice, s);
-  rc = enqueue_pinned_release(s, slot);
-  if (e != cudaSuccess) return record_error(e, "tail H2D");
-  return rc;
 }
 
 int device_sm_count(int dev, int *sms) {

@@ -30,27 +30,20 @@ bool profile_enabled();
 void profile_mark(cudaStream_t s, const char *name);
 void profile_end_call();
 int profile_collect(char *names, int names_len, float *ms, int max);
-// Serial window combination of one MSM on the host: copies the W window
-// sums (device XYZZ) to a pinned slot, runs Horner in a stream-ordered host
-// function and copies the projective result to d_out.  Not used while the
-// stream is being captured.
-int enqueue_host_tail(cudaStream_t s, int group, const void *d_sums, int W, int c, uint64_t *d_out);
-bool host_tail_enabled();
 // Pinned host slots of PINNED_SLOT_BYTES, recycled; enqueue_pinned_release
 // hands a slot back once the stream reaches that point.
 constexpr size_t PINNED_SLOT_BYTES = 128 * 1024;
 int pinned_acquire(void **p);
 void pinned_release(void *p);
 int enqueue_pinned_release(cudaStream_t s, void *slot);
-void set_host_tail_enabled(bool on);
 // kernel launches issued by this host thread since the last reset
 void count_launches(int k);
 int64_t launches_and_reset();
 int pool_alloc(int dev, cudaStream_t s, size_t bytes, void **ptr);
 int default_window(int group, int64_t n, int limbs);
 
-// Window sums handed to a synchronous caller in place of the stream-ordered
-// host tail: the MSM copies its W window sums (XYZZ, device layout) to
+// Window sums handed to a synchronous caller in place of the device
+// combination: the MSM copies its W window sums (XYZZ, device layout) to
 // `host` (pinned, `cap` bytes), sets W and c and writes no result; the caller
 // combines them (gm_host::horner_to_proj) after synchronising the stream.
 struct TailHandoff {

@@ -56,10 +56,8 @@ struct MsmLayout {
   RedLayout rl;
 
   // slice_threads: accumulation slices (one per thread of a single wave);
-  // level0_wave / coop_wave: threads of k_red_level0 / k_red_level1 resident
-  // at once
-  void plan(int64_t n_, int limbs, int c, int64_t slice_threads, bool pack, int64_t level0_wave,
-            int64_t coop_wave) {
+  // level0_wave: threads of k_red_level0 resident at once
+  void plan(int64_t n_, int limbs, int c, int64_t slice_threads, bool pack, int64_t level0_wave, int sms) {
     n = n_;
     need_pack = pack;
     dp.c = c;
@@ -80,7 +78,7 @@ struct MsmLayout {
     o_tail = cv.take<xyzz_t<F>>(nthreads);
     o_hk = cv.take<int32_t>(nthreads);
     o_tk = cv.take<int32_t>(nthreads);
-    rl.plan<F>(dp.W, dp.B, level0_wave, cv, coop_wave);
+    rl.plan<F>(dp.W, dp.B, level0_wave, sms, cv);
     long_cap = nthreads / FIX_SHORT + 1;
     o_longq = cv.take<int32_t>((size_t)(1 + long_cap));
     o_err = cv.take<uint32_t>(4);
@@ -162,33 +160,17 @@ static int level0_blocks_per_sm(int dev) {
   return cached[dev];
 }
 
-// Threads of the cooperative level-1 reduction kernel resident at once on
-// the device (cached per device).
-template <class F>
-static int64_t coop_wave_threads(int dev, int sms) {
-  static std::mutex mu;
-  static int cached[64] = {0};
-  std::lock_guard<std::mutex> lk(mu);
-  if (dev < 0 || dev >= 64) dev = 0;
-  if (cached[dev] == 0) {
-    int b = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_red_level1<F>, 128, 0) != cudaSuccess) b = 1;
-    cached[dev] = std::max(1, b);
-  }
-  return (int64_t)sms * cached[dev] * 128;
-}
-
 // Split fix-up: short runs serially, long runs by a block-level tree.
 // long_q[0] must be zero on entry.
 template <class F>
 int fixup_launch(cudaStream_t s, const uint32_t *offsets, int64_t K, int64_t nthreads, xyzz_t<F> *buckets,
                  const xyzz_t<F> *head, const xyzz_t<F> *tail, const int32_t *hk, const int32_t *tk, uint32_t *err,
                  int32_t *long_q, int64_t long_cap, int *launches) {
-  k_fixup_split<F><<<grid_for(nthreads, 128), 128, 0, s>>>(offsets, K, nthreads, buckets, head, tail, hk, tk, err,
-                                                            long_q, long_cap);
+  k_fixup_split<F><<<grid_for(nthreads, W_THREADS / 32), W_THREADS, w_smem_bytes<F>(W_THREADS / 32), s>>>(
+      offsets, K, nthreads, buckets, head, tail, hk, tk, err, long_q, long_cap);
   GM_CHECK_LAUNCH("k_fixup_split");
-  k_fixup_long<F><<<FIX_LONG_BLOCKS, 128, 0, s>>>(offsets, K, nthreads, buckets, head, tail, hk, err, long_q,
-                                                   long_cap);
+  k_fixup_long<F><<<FIX_LONG_BLOCKS, 32 * SUM_WARPS, w_sum_smem<F>(SUM_WARPS), s>>>(offsets, K, nthreads, buckets, head,
+                                                                                    tail, hk, err, long_q, long_cap);
   GM_CHECK_LAUNCH("k_fixup_long");
   *launches += 2;
   return GM_OK;
@@ -201,25 +183,31 @@ int reduce_launch(cudaStream_t s, const RedLayout &rl, const xyzz_t<F> *buckets,
                   const xyzz_t<F> **sums, int *launches) {
   auto *X = (xyzz_t<F> *)(ws + rl.o_X);
   auto *A0 = (xyzz_t<F> *)(ws + rl.o_A0);
-  const int64_t wave = (int64_t)rl.sms * level0_blocks_per_sm<F>(rl.dev);
-  const int64_t blocks0 = std::min<int64_t>(wave, (rl.G * rl.nseg0 + 127) / 128);
-  k_red_level0<F><<<(unsigned)std::max<int64_t>(1, blocks0), 128, 0, s>>>(buckets, offsets, rl.G, rl.B, rl.L0,
-                                                                           rl.nseg0, X, rl.M, A0);
+  constexpr int WPB = W_THREADS / 32;
+  if (rl.warp0) {
+    k_red_level0_warp<F><<<grid_for(rl.G * rl.nseg0, WPB), W_THREADS, w_smem_bytes<F>(WPB), s>>>(
+        buckets, offsets, rl.G, rl.B, rl.L0, rl.nseg0, X, rl.M, A0);
+  } else {
+    const int64_t wave = (int64_t)rl.sms * level0_blocks_per_sm<F>(rl.dev);
+    const int64_t blocks0 = std::min<int64_t>(wave, (rl.G * rl.nseg0 + 127) / 128);
+    k_red_level0<F><<<(unsigned)std::max<int64_t>(1, blocks0), 128, 0, s>>>(buckets, offsets, rl.G, rl.B, rl.L0,
+                                                                             rl.nseg0, X, rl.M, A0);
+  }
   GM_CHECK_LAUNCH("k_red_level0");
   (*launches)++;
   if (rl.nseg1 > 0) {
-    k_red_level1<F><<<grid_for((int64_t)Coop<F>::LANES * rl.G * rl.nseg1, 128), 128, 0, s>>>(A0, rl.G, rl.nseg0, rl.L1, rl.nseg1,
-                                                                        rl.L0, X, rl.M);
+    k_red_level1<F><<<grid_for(rl.G * rl.nseg1, WPB), W_THREADS, w_smem_bytes<F>(WPB), s>>>(
+        A0, rl.G, rl.nseg0, rl.L1, rl.nseg1, rl.L0, X, rl.M);
     GM_CHECK_LAUNCH("k_red_level1");
     (*launches)++;
   }
   const xyzz_t<F> *src = X;
   int N = rl.M, k = 0;
   while (N > 1) {
-    const int nout = (N + RedLayout::FAN - 1) / RedLayout::FAN;
+    const int chunk = RedLayout::sum_chunk(N), nout = (N + chunk - 1) / chunk;
     auto *dst = (xyzz_t<F> *)(ws + rl.o_t[k]);
-    k_tree_quad<F><<<grid_for((int64_t)Coop<F>::LANES * rl.G * nout, 128), 128, 0, s>>>(src, rl.G, N, RedLayout::FAN, dst);
-    GM_CHECK_LAUNCH("k_tree_quad");
+    k_red_sum<F><<<(unsigned)(rl.G * nout), 32 * SUM_WARPS, w_sum_smem<F>(SUM_WARPS), s>>>(src, N, chunk, nout, dst);
+    GM_CHECK_LAUNCH("k_red_sum");
     (*launches)++;
     src = dst;
     k ^= 1;
@@ -245,9 +233,7 @@ int msm_plan(MsmLayout<F> &lay, int dev, int64_t n, int limbs, int c, bool pack,
   int rc = device_sm_count(dev, &sms);
   if (rc) return rc;
   if (slice_threads <= 0) slice_threads = (int64_t)sms * acc_blocks_per_sm<F>(dev) * ACC_THREADS;
-  lay.plan(n, limbs, c, slice_threads, pack, (int64_t)sms * level0_blocks_per_sm<F>(dev) * 128,
-           coop_wave_threads<F>(dev, sms));
-  lay.rl.sms = sms;
+  lay.plan(n, limbs, c, slice_threads, pack, (int64_t)sms * level0_blocks_per_sm<F>(dev) * 128, sms);
   lay.rl.dev = dev;
   if ((uint64_t)n * lay.dp.W >= (1ull << 32)) {
     set_last_error("too many (point, window) entries for 32-bit offsets");
@@ -260,16 +246,14 @@ int msm_plan(MsmLayout<F> &lay, int dev, int64_t n, int limbs, int c, bool pack,
 // (lay.bytes, 256-byte aligned); allocates nothing itself.  bases: packed
 // records, or null to pack from ref_points (reference layout; to_mont converts
 // standard-form points).  out_proj receives the projective result in the
-// reference layout.  host_tail: the window combination runs on the host (a
-// pinned staging slot and a stream-ordered host function); otherwise, and
-// always while s is being captured, on the device.  err_out (optional,
+// reference layout.  err_out (optional,
 // device) receives the consistency flag of the fix-up (0 = ok).  bases_ready
 // (optional): an event the stream waits for after the sort, before the bases
 // are first read.  handoff (optional): the window sums are copied to the
 // caller's pinned buffer instead, and out_proj is not written.
 template <class F>
 int msm_run(cudaStream_t s, const MsmLayout<F> &lay, char *ws, const uint4 *bases, const uint64_t *ref_points,
-            int to_mont, const uint64_t *scalars, uint64_t *out_proj, bool host_tail, uint32_t *err_out,
+            int to_mont, const uint64_t *scalars, uint64_t *out_proj, uint32_t *err_out,
             cudaEvent_t bases_ready, TailHandoff *handoff = nullptr) {
   constexpr int H = F::LIMBS / 2;  // u64 words per coordinate
   const int64_t n = lay.n;
@@ -314,21 +298,19 @@ int msm_run(cudaStream_t s, const MsmLayout<F> &lay, char *ws, const uint4 *base
   if (rc) return rc;
   profile_mark(s, "fixup");
 
-  // bucket reduction: leveled running sums, then a quad fan-in tree
+  // bucket reduction: leveled running sums, then block sums
   const int W = lay.dp.W;
   const xyzz_t<F> *src = nullptr;
   rc = reduce_launch<F>(s, lay.rl, buckets, offsets, ws, &src, &launches);
   if (rc) return rc;
   profile_mark(s, "reduce");
-  // window combination: the serial Horner tail runs on the host (lower
-  // latency per product) unless the stream is being captured into a graph
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  GM_CHECK(cudaStreamIsCapturing(s, &cap));
-  if (handoff && cap != cudaStreamCaptureStatusNone) {
-    set_last_error("window-sum handoff while the stream is being captured");
-    return GM_ERR_ARG;
-  }
   if (handoff) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    GM_CHECK(cudaStreamIsCapturing(s, &cap));
+    if (cap != cudaStreamCaptureStatusNone) {
+      set_last_error("window-sum handoff while the stream is being captured");
+      return GM_ERR_ARG;
+    }
     const size_t bytes = (size_t)W * sizeof(xyzz_t<F>);
     if (bytes > handoff->cap) {
       set_last_error("window-sum handoff buffer too small");
@@ -337,12 +319,9 @@ int msm_run(cudaStream_t s, const MsmLayout<F> &lay, char *ws, const uint4 *base
     GM_CHECK(cudaMemcpyAsync(handoff->host, src, bytes, cudaMemcpyDeviceToHost, s));
     handoff->W = W;
     handoff->c = lay.dp.c;
-  } else if (host_tail && cap == cudaStreamCaptureStatusNone) {
-    rc = enqueue_host_tail(s, F::LIMBS == NL ? 1 : 2, src, W, lay.dp.c, out_proj);
-    if (rc) return rc;
   } else {
-    k_combine_quad<F><<<1, 32, 0, s>>>(src, 1, W, lay.dp.c, nullptr, out_proj);
-    GM_CHECK_LAUNCH("k_combine_quad");
+    k_combine<F><<<1, 32 * COMBINE_WARPS, w_sum_smem<F>(COMBINE_WARPS), s>>>(src, W, lay.dp.c, nullptr, out_proj);
+    GM_CHECK_LAUNCH("k_combine");
     launches++;
   }
   profile_mark(s, "combine");
@@ -371,7 +350,7 @@ int msm_launch(cudaStream_t s, int dev, const uint4 *bases, const uint64_t *ref_
   char *ws = nullptr;
   rc = pool_alloc(dev, s, lay.bytes, (void **)&ws);
   if (rc) return rc;
-  rc = msm_run<F>(s, lay, ws, bases, ref_points, to_mont, scalars, out_proj, host_tail_enabled(), err_out,
+  rc = msm_run<F>(s, lay, ws, bases, ref_points, to_mont, scalars, out_proj, err_out,
                   bases_ready, handoff);
   const cudaError_t e = cudaFreeAsync(ws, s);
   if (rc) return rc;

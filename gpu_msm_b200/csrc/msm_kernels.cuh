@@ -16,9 +16,9 @@
 //  5. k_fixup_*    the slice that opened a straddling bucket adds the
 //                  partials of the following slices (msm_reduce.cuh).
 //  6. k_red_*      per window, sum_b (b+1)*Bucket_b by segmented running sums
-//                  and a quad fan-in tree (msm_reduce.cuh).
-//  7. combine      result = sum_w 2^(c*w) * S_w by Horner (host tail, or
-//                  k_combine_quad on the device), converted to the
+//                  and block sums (msm_reduce.cuh).
+//  7. combine      result = sum_w 2^(c*w) * S_w by Horner
+//                  (k_combine), converted to the
 //                  reference's homogeneous projective output.
 //
 // Packed base records (written once by k_pack_*): affine x, y in Montgomery

@@ -38,7 +38,7 @@ namespace gm {
 // instantiated once, in msm_g1.cu
 extern template int msm_plan<Fp>(MsmLayout<Fp> &, int, int64_t, int, int, bool, int64_t);
 extern template int msm_run<Fp>(cudaStream_t, const MsmLayout<Fp> &, char *, const uint4 *, const uint64_t *, int,
-                                const uint64_t *, uint64_t *, bool, uint32_t *, cudaEvent_t, TailHandoff *);
+                                const uint64_t *, uint64_t *, uint32_t *, cudaEvent_t, TailHandoff *);
 }  // namespace gm
 
 namespace {
@@ -107,8 +107,7 @@ extern "C" int gm_g1_msm_device_noalloc(gm_stream_t stream, uint32_t gpu_index, 
     gm::set_last_error("gm_g1_msm_device_noalloc: request exceeds the fixed scratch size");
     return gm::GM_ERR_ARG;
   }
-  // the same pipeline as the regular entry points, in the fixed array, with
-  // the window combination on the device (the host tail needs pinned memory)
+  // the same pipeline as the regular entry points, in the fixed array
   return gm::msm_run<Fp>(s, lay, static_cast<char *>(base), nullptr, (const uint64_t *)d_points, 0, d_scalars,
-                         (uint64_t *)d_result, /*host_tail=*/false, d_err, nullptr);
+                         (uint64_t *)d_result, d_err, nullptr);
 }

@@ -8,22 +8,28 @@
 //     T_s = sum_r (r + 1) V_{s L0 + r},   A_s = sum_r V_{s L0 + r},
 // two additions per bucket and nothing else.  Then
 //     S_g = sum_s T_s + L0 * sum_s s A_s.
-// Level 1 cuts the A_s into segments of L1; a cooperative group of lanes
-// (coop.cuh) per segment s' computes  D = sum_r r A_{s' L1 + r},  A' = sum_r A_{s' L1 + r}  and
+// Level 1 cuts the A_s into segments of L1; a warp per segment s' computes  D = sum_r r A_{s' L1 + r},  A' = sum_r A_{s' L1 + r}  and
 //     E_{s'} = L0 * (D + (s' L1) A')          (double-and-add, then doublings)
 // so that  sum_s s A_s = sum_{s'} (D + s' L1 A')  and
 //     S_g = sum_s T_s + sum_{s'} E_{s'}.
-// A cooperative fan-in tree adds the nseg0 + nseg1 values of every group.
-// Level 0 is throughput-bound (it holds nearly all the work and enough
-// threads to fill the GPU); the few, serial additions of level 1 and the tree
-// run on quads to cut their latency.  This replaces the reference's per-block
+// Block sums add the nseg0 + nseg1 values of every group.  Level 0 holds
+// nearly all the work; the few, serial additions of level 1 and the sums run
+// on warps (xyzz_warp.cuh) to cut their latency.  B200, against four lanes of
+// one product each: G1 1024 points 0.92 -> 0.07 ms, G1 2^20 2.01 -> 1.56 ms,
+// G2 2^18 3.94 -> 2.87 ms for the whole reduction.  This replaces the reference's per-block
 // partial buckets and per-window host combine (src/curve.cu:1557-1654,
 // :2060-2179) with work that stays on the device.
 #pragma once
 #include "msm_kernels.cuh"
-#include "coop.cuh"
+#include "xyzz_warp.cuh"
 
 namespace gm {
+
+constexpr int W_THREADS = 128;    // block of the kernels with one warp per work item
+constexpr int SUM_WARPS = 8;      // warps of a block sum
+constexpr int COMBINE_WARPS = 8;  // warps of a window combination
+constexpr int W_FILL = 16;        // warps per SM that keep its schedulers busy with dependent point operations
+constexpr int RED_THREAD_MIN = 3;  // level 0 goes to threads above this many buckets per thread of a wave
 
 // Level 0: segments (group, s) in a grid-stride loop.  The host picks L0 so
 // that all segments fit in one resident wave when it can (no partial second
@@ -64,48 +70,64 @@ __global__ void __launch_bounds__(128) k_red_level0(const xyzz_t<F> *__restrict_
   }
 }
 
-// Level 1: one cooperative group of lanes per (group, segment s').  Writes E_{s'} to X[g*M + nseg0 + s'].
+// Level 0 on warps (warp_field.cuh): one warp per segment.  A segment's two
+// additions per bucket are one serial chain, 40 us per bucket in one thread
+// and 2.6 us in a warp (G1), so warps take over wherever the segments do not
+// fill the GPU with threads (RedLayout::plan has the rule).
 template <class F>
-__global__ void __launch_bounds__(128) k_red_level1(const xyzz_t<F> *__restrict__ A0, int64_t G, int nseg0, int L1,
-                                                    int nseg1, int L0, xyzz_t<F> *__restrict__ X, int M) {
-  using C = Coop<F>;
-  using FA = typename C::A;
-  const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / C::LANES;
+__global__ void __launch_bounds__(W_THREADS) k_red_level0_warp(const xyzz_t<F> *__restrict__ buckets,
+                                                               const uint32_t *__restrict__ offsets, int64_t G, int B,
+                                                               int L0, int nseg0, xyzz_t<F> *__restrict__ X, int M,
+                                                               xyzz_t<F> *__restrict__ A0) {
+  w_setup();
+  const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (t >= G * nseg0) return;
+  const int64_t g = t / nseg0;
+  const int s = (int)(t % nseg0);
+  const int64_t kb = g * B;
+  wpt<F> acc = w_inf<F>(), ws = w_inf<F>();
+  const int j0 = s * L0, j1 = min(B, j0 + L0);
+  for (int j = j1 - 1; j >= j0; j--) {
+    if (__ldg(offsets + kb + j + 1) != __ldg(offsets + kb + j)) acc = w_addp<F>(acc, w_load_pt<F>(buckets + kb + j));
+    ws = w_addp<F>(ws, acc);
+  }
+  w_store_pt<F>(X + g * M + s, ws);
+  w_store_pt<F>(A0 + g * nseg0 + s, acc);
+}
+
+// Level 1: one warp per (group, segment s').  Writes E_{s'} to X[g*M + nseg0 + s'].
+template <class F>
+__global__ void __launch_bounds__(W_THREADS) k_red_level1(const xyzz_t<F> *__restrict__ A0, int64_t G, int nseg0,
+                                                          int L1, int nseg1, int L0, xyzz_t<F> *__restrict__ X, int M) {
+  w_setup();
+  const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (t >= G * nseg1) return;
   const int64_t g = t / nseg1;
   const int s = (int)(t % nseg1);
   const int r0 = s * L1, r1 = min(nseg0, r0 + L1);
-  xyzz_t<FA> acc, ws;
-  xyzz_set_inf(acc);
-  xyzz_set_inf(ws);
+  wpt<F> acc = w_inf<F>(), ws = w_inf<F>();
   for (int r = r1 - 1; r >= r0; r--) {
-    C::add(acc, as_xyzz<FA>(A0[g * nseg0 + r]));
-    if (r > r0) C::add(ws, acc);
+    acc = w_addp<F>(acc, w_load_pt<F>(A0 + g * nseg0 + r));
+    if (r > r0) ws = w_addp<F>(ws, acc);
   }
   // ws = sum (r - r0) A_r; add (s L1) * acc, then scale by L0
-  xyzz_t<FA> m;
-  coop_mul_small<F>(m, acc, (uint32_t)r0);
-  C::add(ws, m);
-  coop_mul_small<F>(m, ws, (uint32_t)L0);
-  if (coop_leader<F>()) X[g * M + nseg0 + s] = as_xyzz<F>(m);
+  ws = w_addp<F>(ws, w_mul_small<F>(acc, (uint32_t)r0));
+  w_store_pt<F>(X + g * M + nseg0 + s, w_mul_small<F>(ws, (uint32_t)L0));
 }
 
-// out[g*nout + i] = sum_{k < fan} in[g*N + i*fan + k], one cooperative
-// group per output
+// out[g*nout + i] = sum of in[g*N + j], j in [i*chunk, (i+1)*chunk): one block
+// of SUM_WARPS warps per output, strided sums and a tree in shared memory.
 template <class F>
-__global__ void __launch_bounds__(128) k_tree_quad(const xyzz_t<F> *__restrict__ in, int64_t G, int N, int fan,
-                                                   xyzz_t<F> *__restrict__ out) {
-  using C = Coop<F>;
-  using FA = typename C::A;
-  const int nout = (N + fan - 1) / fan;
-  const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / C::LANES;
-  if (t >= G * nout) return;
-  const int64_t g = t / nout;
-  const int i = (int)(t % nout);
-  const int64_t base = g * N + (int64_t)i * fan;
-  xyzz_t<FA> acc = as_xyzz<FA>(in[base]);
-  for (int k = 1; k < fan && i * fan + k < N; k++) C::add(acc, as_xyzz<FA>(in[base + k]));
-  if (coop_leader<F>()) out[t] = as_xyzz<F>(acc);
+__global__ void __launch_bounds__(32 * SUM_WARPS) k_red_sum(const xyzz_t<F> *__restrict__ in, int N, int chunk,
+                                                            int nout, xyzz_t<F> *__restrict__ out) {
+  w_setup();
+  const int64_t g = blockIdx.x / nout;
+  const int i = (int)(blockIdx.x % nout);
+  const int j1 = min(N, (i + 1) * chunk);
+  wpt<F> acc = w_inf<F>();
+  for (int j = i * chunk + (threadIdx.x >> 5); j < j1; j += SUM_WARPS) acc = w_addp<F>(acc, w_load_pt<F>(in + g * N + j));
+  acc = w_block_sum<F>(acc, SUM_WARPS, w_smem + w_smem_bytes<F>(SUM_WARPS) / 4);
+  if (threadIdx.x < 32) w_store_pt<F>(out + blockIdx.x, acc);
 }
 
 // ---------------------------------------------------------------------------
@@ -114,125 +136,133 @@ __global__ void __launch_bounds__(128) k_tree_quad(const xyzz_t<F> *__restrict__
 // (part_head).  Runs of at most FIX_SHORT heads are folded serially by the
 // owner of the tail; longer runs (a bucket much larger than a slice, e.g. all
 // the scalars equal to 1) are queued and folded by k_fixup_long, one block of
-// cooperative groups per run with a shared-memory tree.
+// SUM_WARPS warps per run with a shared-memory tree.
 // ---------------------------------------------------------------------------
 constexpr int FIX_SHORT = 8;
 constexpr int FIX_LONG_BLOCKS = 64;
 
 // long_q: [0] = count, then bucket keys
 template <class F>
-__global__ void __launch_bounds__(128) k_fixup_split(const uint32_t *__restrict__ offsets, int64_t K, int64_t nthreads,
-                                                     xyzz_t<F> *__restrict__ buckets,
-                                                     const xyzz_t<F> *__restrict__ part_head,
-                                                     const xyzz_t<F> *__restrict__ part_tail,
-                                                     const int32_t *__restrict__ head_key,
-                                                     const int32_t *__restrict__ tail_key, uint32_t *__restrict__ err,
-                                                     int32_t *__restrict__ long_q, int64_t long_cap) {
-  const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= nthreads) return;
-  const int32_t k = tail_key[t];
+__global__ void __launch_bounds__(W_THREADS) k_fixup_split(const uint32_t *__restrict__ offsets, int64_t K,
+                                                           int64_t nslices, xyzz_t<F> *__restrict__ buckets,
+                                                           const xyzz_t<F> *__restrict__ part_head,
+                                                           const xyzz_t<F> *__restrict__ part_tail,
+                                                           const int32_t *__restrict__ head_key,
+                                                           const int32_t *__restrict__ tail_key,
+                                                           uint32_t *__restrict__ err, int32_t *__restrict__ long_q,
+                                                           int64_t long_cap) {
+  w_setup();
+  const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (t >= nslices) return;
+  const int32_t k = __ldg(tail_key + t);
   if (k < 0) return;
   const uint32_t M = __ldg(offsets + K);
-  const uint64_t chunk64 = ((uint64_t)M + nthreads - 1) / nthreads;
+  const uint64_t chunk64 = ((uint64_t)M + nslices - 1) / nslices;
   const uint64_t chunk = chunk64 > 0 ? chunk64 : 1u;
   const uint64_t bend = __ldg(offsets + k + 1);
   const int64_t t1 = (int64_t)((bend - 1) / chunk);  // slice holding the bucket's last entry
+  const bool lead = (threadIdx.x & 31u) == 0;
   if (t1 - t > FIX_SHORT) {
-    const int32_t slot = atomicAdd(long_q, 1);
-    if (slot < long_cap)
-      long_q[1 + slot] = k;
-    else
-      atomicOr(err, 2u);
+    if (lead) {
+      const int32_t slot = atomicAdd(long_q, 1);
+      if (slot < long_cap)
+        long_q[1 + slot] = k;
+      else
+        atomicOr(err, 2u);
+    }
     return;
   }
-  using FA = typename OutOfLine<F>::type;
-  xyzz_t<FA> acc = as_xyzz<FA>(part_tail[t]);
-  for (int64_t t2 = t + 1; t2 <= t1 && t2 < nthreads; t2++) {
-    if (head_key[t2] != k) {  // cannot happen for a consistent slicing
-      atomicOr(err, 1u);
+  wpt<F> acc = w_load_pt<F>(part_tail + t);
+  for (int64_t t2 = t + 1; t2 <= t1 && t2 < nslices; t2++) {
+    if (__ldg(head_key + t2) != k) {  // cannot happen for a consistent slicing
+      if (lead) atomicOr(err, 1u);
       break;
     }
-    xyzz_add_cold<FA>(acc, as_xyzz<FA>(part_head[t2]));
+    acc = w_addp<F>(acc, w_load_pt<F>(part_head + t2));
   }
-  buckets[k] = as_xyzz<F>(acc);
+  w_store_pt<F>(buckets + k, acc);
 }
 
 template <class F>
-__global__ void __launch_bounds__(128) k_fixup_long(const uint32_t *__restrict__ offsets, int64_t K, int64_t nthreads,
-                                                    xyzz_t<F> *__restrict__ buckets,
-                                                    const xyzz_t<F> *__restrict__ part_head,
-                                                    const xyzz_t<F> *__restrict__ part_tail,
-                                                    const int32_t *__restrict__ head_key, uint32_t *__restrict__ err,
-                                                    const int32_t *__restrict__ long_q, int64_t long_cap) {
-  using C = Coop<F>;
-  using FA = typename C::A;
-  constexpr int GROUPS = 128 / C::LANES;  // cooperative groups per block
-  __shared__ xyzz_t<F> part[GROUPS];
-  const int grp = threadIdx.x / C::LANES;
-  const bool leader = coop_leader<F>();
+__global__ void __launch_bounds__(32 * SUM_WARPS) k_fixup_long(const uint32_t *__restrict__ offsets, int64_t K,
+                                                               int64_t nslices, xyzz_t<F> *__restrict__ buckets,
+                                                               const xyzz_t<F> *__restrict__ part_head,
+                                                               const xyzz_t<F> *__restrict__ part_tail,
+                                                               const int32_t *__restrict__ head_key,
+                                                               uint32_t *__restrict__ err,
+                                                               const int32_t *__restrict__ long_q, int64_t long_cap) {
   const int64_t n_long = min((int64_t)long_q[0], long_cap);
+  if ((int64_t)blockIdx.x >= n_long) return;
+  w_setup();
+  const int w = threadIdx.x >> 5;
   const uint32_t M = __ldg(offsets + K);
-  const uint64_t chunk64 = ((uint64_t)M + nthreads - 1) / nthreads;
+  const uint64_t chunk64 = ((uint64_t)M + nslices - 1) / nslices;
   const uint64_t chunk = chunk64 > 0 ? chunk64 : 1u;
   for (int64_t item = blockIdx.x; item < n_long; item += gridDim.x) {
     const int32_t k = long_q[1 + item];
     const int64_t t0 = (int64_t)(__ldg(offsets + k) / chunk);
-    const int64_t t1 = min((int64_t)((__ldg(offsets + k + 1) - 1) / chunk), nthreads - 1);
-    // group j folds run positions j, j+GROUPS, ... (position 0 is the tail piece)
-    xyzz_t<FA> acc;
-    xyzz_set_inf(acc);
-    for (int64_t p = grp; p <= t1 - t0; p += GROUPS) {
+    const int64_t t1 = min((int64_t)((__ldg(offsets + k + 1) - 1) / chunk), nslices - 1);
+    // warp w folds run positions w, w + SUM_WARPS, ... (position 0 is the tail piece)
+    wpt<F> acc = w_inf<F>();
+    for (int64_t p = w; p <= t1 - t0; p += SUM_WARPS) {
       const int64_t ts = t0 + p;
       if (p == 0) {
-        C::add(acc, as_xyzz<FA>(part_tail[ts]));
-      } else if (head_key[ts] != k) {
-        if (leader) atomicOr(err, 1u);
+        acc = w_addp<F>(acc, w_load_pt<F>(part_tail + ts));
+      } else if (__ldg(head_key + ts) != k) {
+        if ((threadIdx.x & 31u) == 0) atomicOr(err, 1u);
       } else {
-        C::add(acc, as_xyzz<FA>(part_head[ts]));
+        acc = w_addp<F>(acc, w_load_pt<F>(part_head + ts));
       }
     }
-    if (leader) part[grp] = as_xyzz<F>(acc);
-    __syncthreads();
-    for (int h = GROUPS / 2; h >= 1; h >>= 1) {
-      if (grp < h) C::add(acc, as_xyzz<FA>(part[grp + h]));
-      __syncthreads();
-      if (grp < h && leader) part[grp] = as_xyzz<F>(acc);
-      __syncthreads();
-    }
-    if (threadIdx.x == 0) buckets[k] = part[0];
+    acc = w_block_sum<F>(acc, SUM_WARPS, w_smem + w_smem_bytes<F>(SUM_WARPS) / 4);
+    if (w == 0) w_store_pt<F>(buckets + k, acc);
     __syncthreads();
   }
 }
 
 // ---------------------------------------------------------------------------
-// Window combination on the device, one cooperative group per MSM: result = sum_w
-// 2^(c w) S_w by Horner; homogeneous projective output (u64 limbs,
-// Montgomery).  out_index (optional) maps MSM i to its result slot.
+// Window combination on the device, one block of COMBINE_WARPS warps per MSM:
+// result = sum_w 2^(c w) S_w by Horner; homogeneous projective output (u64
+// limbs, Montgomery).  The c (W - 1) doublings of the top window are one
+// serial chain, about 0.9 us each; the additions are kept off it: every warp
+// combines W / COMBINE_WARPS windows, all at once, and warp 0 the warps'
+// sums.  out_index (optional) maps MSM i to its result slot.
 // ---------------------------------------------------------------------------
 template <class F>
-__global__ void __launch_bounds__(128) k_combine_quad(const xyzz_t<F> *__restrict__ S, int n_msm, int W, int c,
-                                                      const int32_t *__restrict__ out_index,
-                                                      uint64_t *__restrict__ out_proj) {
-  using C = Coop<F>;
-  using FA = typename C::A;
-  const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / C::LANES);
-  if (i >= n_msm) return;
-  xyzz_t<FA> res;
-  xyzz_set_inf(res);
-  for (int w = W - 1; w >= 0; w--) {
-    if (!xyzz_is_inf(res))
-      for (int k = 0; k < c; k++) C::dbl(res);
-    C::add(res, as_xyzz<FA>(S[(int64_t)i * W + w]));
+__global__ void __launch_bounds__(32 * COMBINE_WARPS) k_combine(const xyzz_t<F> *__restrict__ S, int W, int c,
+                                                                const int32_t *__restrict__ out_index,
+                                                                uint64_t *__restrict__ out_proj) {
+  using WP = WF<F>;
+  w_setup();
+  const int64_t i = blockIdx.x;
+  const int w = threadIdx.x >> 5;
+  const int q = (W + COMBINE_WARPS - 1) / COMBINE_WARPS;
+  int32_t *sums = w_smem + w_smem_bytes<F>(COMBINE_WARPS) / 4;
+  wpt<F> res = w_inf<F>();
+  for (int j = min(W, (w + 1) * q) - 1; j >= w * q; j--) {
+    if (!res.inf)
+      for (int k = 0; k < c; k++) res = w_dbl<F>(res);
+    res = w_addp<F>(res, w_load_pt<F>(S + i * W + j));
   }
-  if (!coop_leader<F>()) return;
-  typename F::T Xp, Yp, Zp;
-  xyzz_to_proj<FA>(Xp, Yp, Zp, res);
-  constexpr int H = F::LIMBS / 2;
-  const int64_t slot = out_index ? (int64_t)__ldg(out_index + i) : (int64_t)i;
-  uint64_t *o = out_proj + slot * 3 * H;
-  store_ref<F>(o, Xp);
-  store_ref<F>(o + H, Yp);
-  store_ref<F>(o + 2 * H, Zp);
+  w_put_pt<F>(sums + w * w_pt_words<F>(), res);
+  __syncthreads();
+  if (w > 0) return;
+  res = w_get_pt<F>(sums + (COMBINE_WARPS - 1) * w_pt_words<F>());
+  for (int j = COMBINE_WARPS - 2; j >= 0; j--) {
+    if (!res.inf)
+      for (int k = 0; k < c * q; k++) res = w_dbl<F>(res);
+    res = w_addp<F>(res, w_get_pt<F>(sums + j * w_pt_words<F>()));
+  }
+  // (X ZZZ, Y ZZ, ZZ ZZZ); infinity is (0, 0, 0)
+  if (res.inf) res = w_inf<F>();
+  const int g = w_group();
+  const typename F::T o =
+      WP::canon(WP::mul(WP::pick(g, res.X, res.Y, res.ZZ, res.ZZ), WP::pick(g, res.ZZZ, res.ZZ, res.ZZZ, res.ZZZ)));
+  if (g < 3 && w_lane() == 0) {
+    typename F::T v = o;
+    const int64_t slot = out_index ? (int64_t)__ldg(out_index + i) : i;
+    store_ref<F>(out_proj + (slot * 3 + g) * (F::LIMBS / 2), v);
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -242,40 +272,48 @@ struct RedLayout {
   int64_t G = 0;
   int sms = 1, dev = 0;  // device the level-0 grid is sized for
   int B = 0, L0 = 0, nseg0 = 0, L1 = 0, nseg1 = 0, M = 0;
-  static constexpr int FAN = 2;
+  bool warp0 = false;    // level 0 on warps
   size_t o_X = 0, o_A0 = 0, o_t[2] = {0, 0};
 
-  // wave_threads: level-0 threads resident at once on the device.  L0 is at
-  // least 16 buckets for G1 and 4 for G2 (an Fp2 addition takes three times
-  // as long, so G2 wants shorter chains), and larger when the segments would
-  // not fit one wave.  coop_wave: threads of the cooperative level-1 kernel
-  // resident at once (0: no limit); L1 is at least 4 or 8 segments (below),
-  // and larger when the level-1 groups (Coop<F>::LANES threads each) would
-  // not fit one wave: a second wave would double the level's serial time.
+  // values per output of a sum stage over N values per group: up to 64 in one
+  // block (8 additions per warp and the tree), else two stages of about sqrt(N)
+  static int sum_chunk(int N) {
+    if (N <= 64) return N;
+    int q = 1;
+    while (q * q < N) q++;
+    return q;
+  }
+
+  // wave_threads: level-0 threads resident at once on the device.
   template <class F, class Carver>
-  void plan(int64_t G_, int B_, int64_t wave_threads, Carver &cv, int64_t coop_wave = 0) {
+  void plan(int64_t G_, int B_, int64_t wave_threads, int sms_, Carver &cv) {
     G = G_;
     B = B_;
-    int64_t l0 = sizeof(typename F::T) == sizeof(fp_t) ? 16 : 4;
-    if (wave_threads > 0) l0 = std::max<int64_t>(l0, (G * B + wave_threads - 1) / wave_threads);
+    sms = sms_;
+    // Level 0: on warps, about W_FILL warps per SM (they then fill its
+    // schedulers), at least 4 buckets each; on threads when a resident wave of
+    // threads would get more than RED_THREAD_MIN buckets each.
+    const int64_t total = G * B;
+    warp0 = wave_threads <= 0 || total <= RED_THREAD_MIN * wave_threads;
+    int64_t l0;
+    if (warp0)
+      l0 = std::max<int64_t>(4, (total + (int64_t)sms * W_FILL - 1) / ((int64_t)sms * W_FILL));
+    else
+      l0 = (total + wave_threads - 1) / wave_threads;
     L0 = (int)std::min<int64_t>(l0, B);
     nseg0 = (B + L0 - 1) / L0;
-    // 4 segments when the groups of 4-segment runs fill at most half a wave
-    // (more and shorter chains; 2^16 MSMs: G2 reduction 2.01 -> 1.75 ms, G1
-    // 1.28 -> 1.18 ms), else 8 (with 4 the groups of G1 2^20 / G2 2^18 fill
-    // the wave, and their reductions measured 2.05 / 4.45 ms against 2.00 /
-    // 3.94 ms)
-    int64_t l1 = 8;
-    if (coop_wave > 0 && G * nseg0 * Coop<F>::LANES / 4 <= coop_wave / 2) l1 = 4;
-    if (coop_wave > 0) l1 = std::max<int64_t>(l1, (G * nseg0 * Coop<F>::LANES + coop_wave - 1) / coop_wave);
+    const int64_t l1 = std::max<int64_t>(4, (G * nseg0 + (int64_t)sms * W_FILL - 1) / ((int64_t)sms * W_FILL));
     L1 = (int)std::min<int64_t>(l1, nseg0);
     nseg1 = nseg0 > 1 ? (nseg0 + L1 - 1) / L1 : 0;
     M = nseg0 + nseg1;
     o_X = cv.template take<xyzz_t<F>>((size_t)(G * M));
     o_A0 = cv.template take<xyzz_t<F>>((size_t)(G * nseg0));
-    const int64_t t1 = G * ((M + FAN - 1) / FAN);
-    o_t[0] = cv.template take<xyzz_t<F>>((size_t)std::max<int64_t>(1, t1));
-    o_t[1] = cv.template take<xyzz_t<F>>((size_t)std::max<int64_t>(1, (t1 + FAN - 1) / FAN + G));
+    int N = M;
+    for (int k = 0; k < 2; k++) {
+      const int ch = sum_chunk(N);
+      N = (N + ch - 1) / ch;
+      o_t[k] = cv.template take<xyzz_t<F>>((size_t)(G * N));
+    }
   }
 };
 

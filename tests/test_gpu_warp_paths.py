@@ -1,0 +1,59 @@
+"""GPU: the warp-cooperative point arithmetic behind the fix-up, the bucket
+reduction and the window combination, at the sizes where its kernels change
+shape: one and few windows, the most windows, segments that do not divide the
+buckets, sums of one and of two stages, level 0 on warps and on threads; and
+points of order 2, whose double is infinity.  Exact: results are compared as
+canonical affine points."""
+import numpy as np
+import pytest
+import torch
+
+import gpu_msm_b200 as gm
+import oracle
+from gpu_msm_b200 import workload as wl
+
+pytestmark = pytest.mark.gpu
+
+
+def dev(a, cuda):
+    return torch.from_numpy(np.ascontiguousarray(a).view(np.int64)).to(cuda)
+
+
+def run(pts, sc, group, cuda, c=0):
+    out = gm.msm_device(pts, dev(sc, cuda), group=group, window_bits=c)
+    torch.cuda.synchronize()
+    return oracle.proj_to_affine(gm.to_numpy_proj(out, group), group)
+
+
+# (group, n, limbs, c): windows 64 limbs / c + 1, buckets 2^(c-1) per window
+SHAPES = [(1, 1, 1, 20), (1, 40, 1, 16), (1, 70, 8, 2), (1, 300, 5, 7), (1, 500, 2, 13), (1, 2000, 1, 18),
+          (1, 900, 5, 14), (2, 1, 1, 18), (2, 33, 8, 3), (2, 200, 5, 6), (2, 400, 1, 15), (2, 300, 5, 13)]
+
+
+@pytest.mark.parametrize("group,n,limbs,c", SHAPES)
+def test_reduction_shapes(cuda, group, n, limbs, c):
+    rng = np.random.default_rng(n + c)
+    logs = wl.make_base_logs(n, seed=n, dup_frac=0.1)
+    sc = rng.integers(0, 2 ** 64, size=(n, limbs), dtype=np.uint64)
+    sc[:: 5] = 0
+    sc[1:: 5] = 1 if limbs == 1 else sc[1:: 5]
+    pts = gm.generator_mul_batch(dev(logs, cuda), group=group)
+    ks, ts = wl.limbs_to_ints(sc), wl.limbs_to_ints(logs)
+    want = oracle.generator_multiple(sum(k * t for k, t in zip(ks, ts)), group=group)
+    assert oracle.same_point(run(pts, sc, group, cuda, c), want)
+
+
+@pytest.mark.parametrize("c", [2, 4, 9])
+@pytest.mark.parametrize("odd", [False, True])
+def test_points_of_order_two(cuda, c, odd):
+    """(-1, 0) on y^2 = x^3 + 1: its multiples are itself and infinity."""
+    n = 37
+    minus_one = (wl.P_MODULUS - (1 << 448)) % wl.P_MODULUS  # -1 in Montgomery form
+    pts = np.zeros((n, gm.G1_WORDS), dtype=np.uint64)
+    pts[:, :7] = wl.int_to_limbs(minus_one, 7)
+    sc = np.random.default_rng(c).integers(0, 2 ** 64, size=(n, 2), dtype=np.uint64)
+    sc[0, 0] = (int(sc[0, 0]) & ~1) + (int(sc[1:, 0].sum(dtype=np.uint64)) + (1 if odd else 0)) % 2
+    got = run(dev(pts, cuda), sc, 1, cuda, c)
+    assert bool(got["infinity"][0]) == (not odd)
+    if odd:
+        assert np.array_equal(got["x"][0], pts[0, :7]) and not got["y"][0].any()
