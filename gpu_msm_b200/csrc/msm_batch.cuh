@@ -22,6 +22,7 @@ struct BatchClassPlan {
   int count = 0;        // MSMs in this class
   int64_t P = 0;        // points in this class
   int64_t K = 0, nthreads = 0;
+  bool warp_acc = false;  // accumulation slices on warps (then outside the queued launch)
   int64_t tilesA = 0;   // pass-A sort tiles (SA_THREADS * sort_ppt points, one MSM each)
   int slice_waves = 1;  // accumulation slices: this many resident waves of threads
   int sort_ppt = SA_PPT;  // pass-A sort tile: points per thread (2, 4 or 8)
@@ -76,9 +77,11 @@ void batch_class_layout(BatchClassPlan &cp, int limbs, int sms, int dev) {
   // precomputed mode: one bucket set per MSM (no window index in the key)
   const int64_t groups = (int64_t)cp.count * (cp.pc_stride ? 1 : cp.dp.W);
   cp.K = groups * cp.dp.B;
-  cp.nthreads = (int64_t)sms * acc_blocks_per_sm<F>(dev) * ACC_THREADS * cp.slice_waves;
   const int64_t max_entries = cp.P * cp.dp.W;
-  if (cp.nthreads > max_entries) cp.nthreads = std::max<int64_t>(1, (max_entries + 127) / 128 * 128);
+  const AccSlices as =
+      acc_slices(max_entries, (int64_t)sms * acc_blocks_per_sm<F>(dev) * ACC_THREADS * cp.slice_waves, sms);
+  cp.nthreads = as.n;
+  cp.warp_acc = as.warp;
   Carve cv;
   cp.o_offsets = cv.take<uint32_t>(cp.K + 1);
   cp.o_entries = cv.take<uint32_t>((size_t)std::max<int64_t>(1, max_entries));
@@ -155,6 +158,16 @@ int batch_class_finish(const BatchClassPlan &cp, cudaStream_t s, uint64_t *resul
   return GM_OK;
 }
 
+template <class F>
+int batch_class_accumulate(const BatchPlan &plan, const BatchClassPlan &cp, cudaStream_t s, int *launches) {
+  ClassBufs<F> cb(cp);
+  acc_launch<F>(cp.warp_acc, s, cp.pc_table ? cp.pc_table : plan.bases, cb.entries, cb.offsets, cp.K, cp.nthreads,
+                cb.buckets, cb.head, cb.tail, cb.hk, cb.tk);
+  GM_CHECK_LAUNCH("k_accumulate");
+  (*launches)++;
+  return GM_OK;
+}
+
 // Enqueue one class's whole pipeline on `s`.
 template <class F>
 int batch_class_run(const BatchPlan &plan, const BatchClassPlan &cp, cudaStream_t s, const uint64_t *scalars,
@@ -163,11 +176,8 @@ int batch_class_run(const BatchPlan &plan, const BatchClassPlan &cp, cudaStream_
   int launches = 0;
   int rc = batch_class_sort<F>(cp, s, scalars, &launches);
   if (rc) return rc;
-  ClassBufs<F> cb(cp);
-  acc_launch<F>(grid_for(cp.nthreads, ACC_THREADS), s, cp.pc_table ? cp.pc_table : plan.bases, cb.entries,
-                cb.offsets, cp.K, cp.nthreads, cb.buckets, cb.head, cb.tail, cb.hk, cb.tk);
-  GM_CHECK_LAUNCH("k_accumulate");
-  launches++;
+  rc = batch_class_accumulate<F>(plan, cp, s, &launches);
+  if (rc) return rc;
   rc = batch_class_finish<F>(cp, s, results, &launches);
   count_launches(launches);
   return rc;
@@ -184,7 +194,7 @@ int batch_queue_setup(BatchPlan &plan) {
     ClassBufs<F> cb(cp);
     h[k] = AccClass<F>{cp.pc_table ? cp.pc_table : plan.bases, cb.entries, cb.offsets, cp.K, cp.nthreads,
                        cb.buckets, cb.head, cb.tail, cb.hk, cb.tk, items};
-    items += cp.nthreads / 32;  // nthreads is a multiple of 128
+    if (!cp.warp_acc) items += cp.nthreads / 32;  // nthreads is a multiple of 128 then
   }
   plan.queue_items = items;
   GM_CHECK(cudaMemcpy(plan.acc_desc, h.data(), h.size() * sizeof(AccClass<F>), cudaMemcpyHostToDevice));
@@ -200,10 +210,20 @@ int batch_run_queued(const BatchPlan &plan, cudaStream_t s, const uint64_t *scal
   GM_CHECK(cudaEventRecord(plan.fork, s));
   for (const auto &cp : plan.classes) {
     GM_CHECK(cudaStreamWaitEvent(cp.stream, plan.fork, 0));
-    const int rc = batch_class_sort<F>(cp, cp.stream, scalars, &launches);
+    int rc = batch_class_sort<F>(cp, cp.stream, scalars, &launches);
     if (rc) return rc;
+    if (cp.warp_acc) {  // few entries: the class's whole pipeline beside the others
+      rc = batch_class_accumulate<F>(plan, cp, cp.stream, &launches);
+      if (rc) return rc;
+      rc = batch_class_finish<F>(cp, cp.stream, results, &launches);
+      if (rc) return rc;
+    }
     GM_CHECK(cudaEventRecord(cp.sorted, cp.stream));
     GM_CHECK(cudaStreamWaitEvent(s, cp.sorted, 0));
+  }
+  if (plan.queue_items == 0) {
+    count_launches(launches);
+    return GM_OK;
   }
   GM_CHECK(cudaMemsetAsync(plan.queue_ctr, 0, sizeof(uint32_t), s));
   int dev = 0, sms = 0;
@@ -217,6 +237,7 @@ int batch_run_queued(const BatchPlan &plan, cudaStream_t s, const uint64_t *scal
   launches++;
   GM_CHECK(cudaEventRecord(plan.acc_done, s));
   for (const auto &cp : plan.classes) {
+    if (cp.warp_acc) continue;
     GM_CHECK(cudaStreamWaitEvent(cp.stream, plan.acc_done, 0));
     rc = batch_class_finish<F>(cp, cp.stream, results, &launches);
     if (rc) return rc;

@@ -44,6 +44,32 @@ struct Carve {
   }
 };
 
+// How the entries of an MSM (or of a batch class) are cut for accumulation.
+// Warps: slices of ACC_WARP_MIN entries, of more once that would give more
+// than W_FILL warps per SM, up to ACC_WARP_MAX entries on 4 times as many.
+// Threads beyond: one slice per thread of a wave, of at least ACC_THREAD_MIN
+// entries (shorter ones leave every bucket to the fix-up).  B200, one slice
+// per thread at all sizes -> this rule, accumulation + fix-up: G1 1024 points
+// 0.24 -> 0.12 ms, G2 1500 points 0.98 -> 0.37 ms, G1 4500 points 0.62 -> 0.30 ms.
+// most: a caller's own bound on the slices (their partials' memory), or 0.
+struct AccSlices {
+  int64_t n = 0;
+  bool warp = false;
+};
+static inline AccSlices acc_slices(int64_t max_entries, int64_t wave_threads, int sms, int64_t most = 0) {
+  AccSlices a;
+  const int64_t warps = (int64_t)sms * W_FILL;
+  if (max_entries <= 4 * warps * ACC_WARP_MAX) {
+    a.warp = true;
+    const int64_t per = std::min<int64_t>(ACC_WARP_MAX, std::max<int64_t>(ACC_WARP_MIN, max_entries / warps));
+    a.n = std::max<int64_t>(1, (max_entries + per - 1) / per);
+  } else {
+    a.n = std::min<int64_t>(std::max<int64_t>(128, wave_threads), (max_entries / ACC_THREAD_MIN + 127) / 128 * 128);
+  }
+  if (most > 0) a.n = std::min(a.n, most);
+  return a;
+}
+
 template <class F>
 struct MsmLayout {
   DigitParams dp;
@@ -52,12 +78,15 @@ struct MsmLayout {
   size_t bytes = 0;
   int64_t long_cap = 0;
   bool need_pack = false;
+  bool warp_acc = false;  // accumulation slices on warps
   SortLayout sl;
   RedLayout rl;
 
   // slice_threads: accumulation slices (one per thread of a single wave);
+  // most_slices: bound on them, or 0;
   // level0_wave: threads of k_red_level0 resident at once
-  void plan(int64_t n_, int limbs, int c, int64_t slice_threads, bool pack, int64_t level0_wave, int sms) {
+  void plan(int64_t n_, int limbs, int c, int64_t slice_threads, bool pack, int64_t level0_wave, int sms,
+            int64_t most_slices) {
     n = n_;
     need_pack = pack;
     dp.c = c;
@@ -65,10 +94,10 @@ struct MsmLayout {
     dp.B = 1 << (c - 1);
     dp.limbs = limbs;
     K = (int64_t)dp.W * dp.B;
-    nthreads = std::max<int64_t>(ACC_THREADS, slice_threads);
-    // never more slices than entries
     const int64_t max_entries = n * dp.W;
-    if (nthreads > max_entries) nthreads = std::max<int64_t>(1, (max_entries + 127) / 128 * 128);
+    const AccSlices as = acc_slices(max_entries, slice_threads, sms, most_slices);
+    nthreads = as.n;
+    warp_acc = as.warp;
     Carve cv;
     o_offsets = cv.take<uint32_t>(K + 1);
     o_entries = cv.take<uint32_t>((size_t)std::max<int64_t>(1, max_entries));
@@ -134,9 +163,16 @@ static int acc_blocks_per_sm(int dev) {
 }
 
 template <class F>
-static void acc_launch(unsigned grid, cudaStream_t s, const uint4 *bases, const uint32_t *entries,
+static void acc_launch(bool warp, cudaStream_t s, const uint4 *bases, const uint32_t *entries,
                        const uint32_t *offsets, int64_t K, int64_t nthreads, xyzz_t<F> *buckets, xyzz_t<F> *head,
                        xyzz_t<F> *tail, int32_t *hk, int32_t *tk) {
+  if (warp) {
+    constexpr int WPB = W_THREADS / 32;
+    k_accumulate_warp<F><<<(unsigned)((nthreads + WPB - 1) / WPB), W_THREADS, w_smem_bytes<F>(WPB), s>>>(
+        bases, entries, offsets, K, nthreads, buckets, head, tail, hk, tk);
+    return;
+  }
+  const unsigned grid = (unsigned)((nthreads + ACC_THREADS - 1) / ACC_THREADS);
   int dev = 0;
   cudaGetDevice(&dev);
   k_accumulate<F><<<grid, ACC_THREADS, acc_occupancy<F>(dev).smem, s>>>(bases, entries, offsets, K, nthreads,
@@ -218,7 +254,8 @@ int reduce_launch(cudaStream_t s, const RedLayout &rl, const xyzz_t<F> *buckets,
 }
 
 // Plans the workspace of one MSM on device dev.  slice_threads 0: one
-// accumulation slice per thread of a full wave (ACC_BLOCKS_MAX blocks per SM).
+// accumulation slice per thread of a full wave (ACC_BLOCKS_MAX blocks per SM)
+// or per warp (acc_slices); else at most that many slices.
 template <class F>
 int msm_plan(MsmLayout<F> &lay, int dev, int64_t n, int limbs, int c, bool pack, int64_t slice_threads) {
   if (limbs < 1 || limbs > MAX_SCALAR_LIMBS || n < 1 || n > (int64_t)INT32_MAX) {
@@ -232,8 +269,9 @@ int msm_plan(MsmLayout<F> &lay, int dev, int64_t n, int limbs, int c, bool pack,
   int sms = 0;
   int rc = device_sm_count(dev, &sms);
   if (rc) return rc;
+  const int64_t most = slice_threads;
   if (slice_threads <= 0) slice_threads = (int64_t)sms * acc_blocks_per_sm<F>(dev) * ACC_THREADS;
-  lay.plan(n, limbs, c, slice_threads, pack, (int64_t)sms * level0_blocks_per_sm<F>(dev) * 128, sms);
+  lay.plan(n, limbs, c, slice_threads, pack, (int64_t)sms * level0_blocks_per_sm<F>(dev) * 128, sms, most);
   lay.rl.dev = dev;
   if ((uint64_t)n * lay.dp.W >= (1ull << 32)) {
     set_last_error("too many (point, window) entries for 32-bit offsets");
@@ -288,8 +326,7 @@ int msm_run(cudaStream_t s, const MsmLayout<F> &lay, char *ws, const uint4 *base
     launches++;
     profile_mark(s, "pack");
   }
-  acc_launch<F>(grid_for(lay.nthreads, ACC_THREADS), s, bases, entries, offsets, lay.K, lay.nthreads, buckets, head,
-                tail, hk, tk);
+  acc_launch<F>(lay.warp_acc, s, bases, entries, offsets, lay.K, lay.nthreads, buckets, head, tail, hk, tk);
   GM_CHECK_LAUNCH("k_accumulate");
   launches++;
   profile_mark(s, "accumulate");

@@ -29,7 +29,81 @@ constexpr int W_THREADS = 128;    // block of the kernels with one warp per work
 constexpr int SUM_WARPS = 8;      // warps of a block sum
 constexpr int COMBINE_WARPS = 8;  // warps of a window combination
 constexpr int W_FILL = 16;        // warps per SM that keep its schedulers busy with dependent point operations
+constexpr int ACC_WARP_MIN = 4;    // entries of a slice on a warp, at least
+constexpr int ACC_WARP_MAX = 16;   // and at most; above W_SLICES slices of these, threads take the slices
+constexpr int ACC_THREAD_MIN = 16;  // entries of a slice on a thread, at least
 constexpr int RED_THREAD_MIN = 3;  // level 0 goes to threads above this many buckets per thread of a wave
+
+// ---------------------------------------------------------------------------
+// Bucket accumulation with one warp per slice, for MSMs with few entries.
+// The slices, partials and outputs are those of k_accumulate.  A mixed
+// addition is a chain of 10 products in one thread, 14 us, and 1.8 us in a
+// warp (G1, B200), but it takes the multiplier of 12 thread additions; so a
+// warp takes the slice while the slices of at least ACC_WARP_MIN entries fit
+// the GPU's schedulers a few times over (acc_slices has the rule).
+// ---------------------------------------------------------------------------
+template <class F>
+__global__ void __launch_bounds__(W_THREADS) k_accumulate_warp(
+    const uint4 *__restrict__ bases, const uint32_t *__restrict__ entries, const uint32_t *__restrict__ offsets,
+    int64_t K, int64_t nslices, xyzz_t<F> *__restrict__ buckets, xyzz_t<F> *__restrict__ part_head,
+    xyzz_t<F> *__restrict__ part_tail, int32_t *__restrict__ head_key, int32_t *__restrict__ tail_key) {
+  using W = WF<F>;
+  using E = typename W::E;
+  w_setup();
+  const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (t >= nslices) return;
+  const uint32_t M = __ldg(offsets + K);
+  const uint64_t chunk64 = ((uint64_t)M + nslices - 1) / nslices;
+  const uint32_t chunk = chunk64 > 0 ? (uint32_t)chunk64 : 1u;
+  const uint64_t start64 = (uint64_t)t * chunk;
+  int32_t hk = -1, tk = -1;
+  if (start64 < M) {
+    const uint32_t end = (uint32_t)(start64 + chunk < M ? start64 + chunk : M);
+    uint32_t pos = (uint32_t)start64;
+    int64_t k = bucket_of(offsets, K, pos);
+    uint32_t bend = __ldg(offsets + k + 1);
+    bool owns = __ldg(offsets + k) == pos;
+    wpt<F> acc = w_inf<F>();
+    uint32_t e = __ldg(entries + pos);
+    const uint32_t *rec = reinterpret_cast<const uint32_t *>(bases + (size_t)(e >> 1) * Rec<F>::U4);
+    typename W::Raw rx = W::fetch(rec), ry = W::fetch(rec + F::LIMBS);
+    while (true) {
+      const E x = W::cut(rx);
+      E y = W::cut(ry);
+      if (e & 1u) y = W::sub(W::zero(), y);
+      if (pos + 1 < end) {  // the next base, on its way during this addition
+        e = __ldg(entries + pos + 1);
+        rec = reinterpret_cast<const uint32_t *>(bases + (size_t)(e >> 1) * Rec<F>::U4);
+        rx = W::fetch(rec);
+        ry = W::fetch(rec + F::LIMBS);
+      }
+      // packed records of the point at infinity hold x = y = 0
+      if (!(W::raw_zero(x) && W::raw_zero(y))) acc = w_madd<F>(acc, x, y);
+      pos++;
+      if (pos == bend || pos == end) {
+        if (!owns) {
+          w_store_pt<F>(part_head + t, acc);
+          hk = (int32_t)k;
+        } else if (pos == bend) {
+          w_store_pt<F>(buckets + k, acc);
+        } else {
+          w_store_pt<F>(part_tail + t, acc);
+          tk = (int32_t)k;
+        }
+        if (pos == end) break;
+        k++;
+        while (__ldg(offsets + k + 1) <= pos) k++;
+        bend = __ldg(offsets + k + 1);
+        owns = true;
+        acc = w_inf<F>();
+      }
+    }
+  }
+  if ((threadIdx.x & 31u) == 0) {
+    head_key[t] = hk;
+    tail_key[t] = tk;
+  }
+}
 
 // Level 0: segments (group, s) in a grid-stride loop.  The host picks L0 so
 // that all segments fit in one resident wave when it can (no partial second

@@ -273,14 +273,21 @@ GM_DEVI void w_redc(wfp (&out)[N], const WCols (&t)[N], int32_t *st) {
   }
 }
 
-// Element in memory (14 words) -> limbs of this lane
-GM_DEVI wfp w_load(const uint32_t *w) {
-  const int l = w_lane();
-  const int j = (7 * l) >> 2, s = (24 * l) & 31;
-  const uint32_t w0 = w[j], w1 = w[j + 1], w2 = w[min(j + 2, NL - 1)];
-  const uint32_t lo = __funnelshift_r(w0, w1, s), hi = __funnelshift_r(w1, w2, s);
+// Element in memory (14 words) -> limbs of this lane: the three words that
+// hold them, and the limbs cut out of these.
+struct wwords {
+  uint32_t w0, w1, w2;
+};
+GM_DEVI wwords w_fetch(const uint32_t *w) {
+  const int j = (7 * w_lane()) >> 2;
+  return wwords{w[j], w[j + 1], w[min(j + 2, NL - 1)]};
+}
+GM_DEVI wfp w_cut(const wwords &v) {
+  const int s = (24 * w_lane()) & 31;
+  const uint32_t lo = __funnelshift_r(v.w0, v.w1, s), hi = __funnelshift_r(v.w1, v.w2, s);
   return wfp{(int32_t)(lo & (uint32_t)WM28), (int32_t)(((lo >> 28) | (hi << 4)) & (uint32_t)WM28)};
 }
+GM_DEVI wfp w_load(const uint32_t *w) { return w_cut(w_fetch(w)); }
 
 // Canonical value (per group; every lane of a group gets it) of |v| < 20 p.
 // st: the group's t slot.
@@ -357,6 +364,9 @@ struct WF<Fp> {
   // difference as a factor of values below 2 p
   GM_DEVI static E diff(const E &a, const E &b) { return w_sub(a, b); }
   GM_DEVI static E mul(const E &a, const E &b) { return w_mul_fp(a, b); }
+  using Raw = wwords;
+  GM_DEVI static Raw fetch(const uint32_t *w) { return w_fetch(w); }
+  GM_DEVI static E cut(const Raw &v) { return w_cut(v); }
   GM_DEVI static E load(const T *p) { return w_load(reinterpret_cast<const uint32_t *>(p)); }
   GM_DEVI static E load_words(const uint32_t *w) { return w_load(w); }
   GM_DEVI static E from(const E &r, int g) {
@@ -381,13 +391,8 @@ struct WF<Fp> {
   }
   static constexpr int LW = 16;  // words of an element in shared memory
   GM_DEVI static E one() {
-    uint32_t w[3];
-    const int l = w_lane();
-    const int j = (7 * l) >> 2, s = (24 * l) & 31;
-#pragma unroll
-    for (int e = 0; e < 3; e++) w[e] = FpConst::ONE(min(j + e, NL - 1));
-    const uint32_t lo = __funnelshift_r(w[0], w[1], s), hi = __funnelshift_r(w[1], w[2], s);
-    return wfp{(int32_t)(lo & (uint32_t)WM28), (int32_t)(((lo >> 28) | (hi << 4)) & (uint32_t)WM28)};
+    const int j = (7 * w_lane()) >> 2;
+    return w_cut(wwords{FpConst::ONE(j), FpConst::ONE(j + 1), FpConst::ONE(min(j + 2, NL - 1))});
   }
 };
 
@@ -433,6 +438,11 @@ struct WF<Fp2> {
   GM_DEVI static E twice(const E &a) { return wfp2{w_carry(w_add(a.c0, a.c0)), w_carry(w_add(a.c1, a.c1))}; }
   GM_DEVI static E diff(const E &a, const E &b) { return sub(a, b); }
   GM_DEVI static E mul(const E &a, const E &b) { return w_mul_fp2(a, b); }
+  struct Raw {
+    wwords c0, c1;
+  };
+  GM_DEVI static Raw fetch(const uint32_t *w) { return Raw{w_fetch(w), w_fetch(w + NL)}; }
+  GM_DEVI static E cut(const Raw &v) { return wfp2{w_cut(v.c0), w_cut(v.c1)}; }
   GM_DEVI static E load(const T *p) { return wfp2{B::load(&p->c0), B::load(&p->c1)}; }
   GM_DEVI static E load_words(const uint32_t *w) { return wfp2{w_load(w), w_load(w + 14)}; }
   GM_DEVI static E from(const E &r, int g) { return wfp2{B::from(r.c0, g), B::from(r.c1, g)}; }

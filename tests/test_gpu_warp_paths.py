@@ -57,3 +57,17 @@ def test_points_of_order_two(cuda, c, odd):
     assert bool(got["infinity"][0]) == (not odd)
     if odd:
         assert np.array_equal(got["x"][0], pts[0, :7]) and not got["y"][0].any()
+
+
+# entries n (64 limbs / c + 1) around the line between slices on warps and on threads of a 148-SM GPU
+# (151552 entries), and far below it
+@pytest.mark.parametrize("group,n,c", [(1, 1, 7), (1, 5, 7), (1, 101, 9), (1, 3294, 7), (1, 3295, 7), (2, 3295, 7)])
+def test_slices_on_warps_and_threads(cuda, group, n, c):
+    """Half of the scalars are equal, so one bucket per window spans many slices; bases repeat and lie at infinity."""
+    logs = wl.make_base_logs(n, seed=n, dup_frac=0.2)
+    logs[::7] = 0
+    sc = wl.make_scalars(n, seed=n + 1)
+    sc[: n // 2] = sc[0]
+    pts = gm.generator_mul_batch(dev(logs, cuda), group=group)
+    want = oracle.generator_multiple(wl.expected_log(sc, logs), group=group)
+    assert oracle.same_point(run(pts, sc, group, cuda, c), want)
