@@ -54,15 +54,15 @@ struct TailHandoff {
 
 // Full MSM pipeline on `s`.  Either `bases` (packed records) or `ref_points`
 // (reference-layout affine points; converted to Montgomery when to_mont) is
-// given.  Writes the projective result (reference layout) to out_proj.  When
+// given.  Writes the result (reference layout; projective, or affine) to out.  When
 // err_out is non-null it receives the device consistency flag (0 = ok).
 // bases_ready (optional): an event the stream waits for after the sort,
 // before the bases are first read (the sort reads only the scalars).
 // handoff (optional, not while capturing): the window sums go to the caller
-// instead of a result in out_proj.
+// instead of a result in out.
 template <class F>
 int msm_launch(cudaStream_t s, int dev, const uint4 *bases, const uint64_t *ref_points, int to_mont,
-               const uint64_t *scalars, int limbs, int64_t n, uint64_t *out_proj, int c_override, uint32_t *err_out,
-               cudaEvent_t bases_ready = nullptr, TailHandoff *handoff = nullptr);
+               const uint64_t *scalars, int limbs, int64_t n, uint64_t *out, int c_override, uint32_t *err_out,
+               cudaEvent_t bases_ready = nullptr, TailHandoff *handoff = nullptr, bool affine = false);
 
 }  // namespace gm

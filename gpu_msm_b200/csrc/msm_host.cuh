@@ -283,16 +283,16 @@ int msm_plan(MsmLayout<F> &lay, int dev, int64_t n, int limbs, int c, bool pack,
 // Enqueues the whole pipeline of one planned MSM on s, in the workspace ws
 // (lay.bytes, 256-byte aligned); allocates nothing itself.  bases: packed
 // records, or null to pack from ref_points (reference layout; to_mont converts
-// standard-form points).  out_proj receives the projective result in the
-// reference layout.  err_out (optional,
+// standard-form points).  out receives the result in the reference layout,
+// projective or (affine) affine.  err_out (optional,
 // device) receives the consistency flag of the fix-up (0 = ok).  bases_ready
 // (optional): an event the stream waits for after the sort, before the bases
 // are first read.  handoff (optional): the window sums are copied to the
-// caller's pinned buffer instead, and out_proj is not written.
+// caller's pinned buffer instead, and out is not written.
 template <class F>
 int msm_run(cudaStream_t s, const MsmLayout<F> &lay, char *ws, const uint4 *bases, const uint64_t *ref_points,
-            int to_mont, const uint64_t *scalars, uint64_t *out_proj, uint32_t *err_out,
-            cudaEvent_t bases_ready, TailHandoff *handoff = nullptr) {
+            int to_mont, const uint64_t *scalars, uint64_t *out, uint32_t *err_out, cudaEvent_t bases_ready,
+            TailHandoff *handoff = nullptr, bool affine = false) {
   constexpr int H = F::LIMBS / 2;  // u64 words per coordinate
   const int64_t n = lay.n;
   auto *offsets = (uint32_t *)(ws + lay.o_offsets);
@@ -357,7 +357,8 @@ int msm_run(cudaStream_t s, const MsmLayout<F> &lay, char *ws, const uint4 *base
     handoff->W = W;
     handoff->c = lay.dp.c;
   } else {
-    k_combine<F><<<1, 32 * COMBINE_WARPS, w_sum_smem<F>(COMBINE_WARPS), s>>>(src, W, lay.dp.c, nullptr, out_proj);
+    k_combine<F><<<1, 32 * COMBINE_WARPS, w_sum_smem<F>(COMBINE_WARPS), s>>>(src, W, lay.dp.c, nullptr, out,
+                                                                                    affine);
     GM_CHECK_LAUNCH("k_combine");
     launches++;
   }
@@ -372,12 +373,13 @@ int msm_run(cudaStream_t s, const MsmLayout<F> &lay, char *ws, const uint4 *base
 // c_override 0: the window width from the cost model.
 template <class F>
 int msm_launch(cudaStream_t s, int dev, const uint4 *bases, const uint64_t *ref_points, int to_mont,
-               const uint64_t *scalars, int limbs, int64_t n, uint64_t *out_proj, int c_override,
-               uint32_t *err_out, cudaEvent_t bases_ready, TailHandoff *handoff) {
+               const uint64_t *scalars, int limbs, int64_t n, uint64_t *out, int c_override,
+               uint32_t *err_out, cudaEvent_t bases_ready, TailHandoff *handoff, bool affine) {
   constexpr int H = F::LIMBS / 2;
   if (n == 0) {
     if (err_out) GM_CHECK(cudaMemsetAsync(err_out, 0, sizeof(uint32_t), s));
-    GM_CHECK(cudaMemsetAsync(out_proj, 0, 3 * H * sizeof(uint64_t), s));
+    GM_CHECK(cudaMemsetAsync(out, 0, (affine ? 2 * H + 1 : 3 * H) * sizeof(uint64_t), s));
+    if (affine) GM_CHECK(cudaMemsetAsync(out + 2 * H, 1, 1, s));  // infinity
     return GM_OK;
   }
   const int c = c_override > 0 ? c_override : default_window(sizeof(typename F::T) == sizeof(fp_t) ? 1 : 2, n, limbs);
@@ -387,8 +389,8 @@ int msm_launch(cudaStream_t s, int dev, const uint4 *bases, const uint64_t *ref_
   char *ws = nullptr;
   rc = pool_alloc(dev, s, lay.bytes, (void **)&ws);
   if (rc) return rc;
-  rc = msm_run<F>(s, lay, ws, bases, ref_points, to_mont, scalars, out_proj, err_out,
-                  bases_ready, handoff);
+  rc = msm_run<F>(s, lay, ws, bases, ref_points, to_mont, scalars, out, err_out, bases_ready,
+                  handoff, affine);
   const cudaError_t e = cudaFreeAsync(ws, s);
   if (rc) return rc;
   return e == cudaSuccess ? GM_OK : record_error(e, "cudaFreeAsync(workspace)");

@@ -300,12 +300,14 @@ __global__ void __launch_bounds__(32 * SUM_WARPS) k_fixup_long(const uint32_t *_
 // limbs, Montgomery).  The c (W - 1) doublings of the top window are one
 // serial chain, about 0.9 us each; the additions are kept off it: every warp
 // combines W / COMBINE_WARPS windows, all at once, and warp 0 the warps'
-// sums.  out_index (optional) maps MSM i to its result slot.
+// sums.  out_index (optional) maps MSM i to its result slot.  affine: an
+// affine point of the reference's layout instead (infinity flag in the word
+// after the coordinates).
 // ---------------------------------------------------------------------------
 template <class F>
 __global__ void __launch_bounds__(32 * COMBINE_WARPS) k_combine(const xyzz_t<F> *__restrict__ S, int W, int c,
                                                                 const int32_t *__restrict__ out_index,
-                                                                uint64_t *__restrict__ out_proj) {
+                                                                uint64_t *__restrict__ out, bool affine) {
   using WP = WF<F>;
   w_setup();
   const int64_t i = blockIdx.x;
@@ -327,15 +329,26 @@ __global__ void __launch_bounds__(32 * COMBINE_WARPS) k_combine(const xyzz_t<F> 
       for (int k = 0; k < c * q; k++) res = w_dbl<F>(res);
     res = w_addp<F>(res, w_get_pt<F>(sums + j * w_pt_words<F>()));
   }
-  // (X ZZZ, Y ZZ, ZZ ZZZ); infinity is (0, 0, 0)
-  if (res.inf) res = w_inf<F>();
+  constexpr int H = F::LIMBS / 2;
   const int g = w_group();
+  const int64_t slot = out_index ? (int64_t)__ldg(out_index + i) : i;
+  if (res.inf) res = w_inf<F>();
+  if (affine) {
+    // x = X ZZZ I, y = Y ZZ I with I = 1 / (ZZ ZZZ); 0 for infinity
+    const typename WP::E I = WP::inv(WP::mul(res.ZZ, res.ZZZ));
+    const typename WP::E t = WP::mul(WP::pick(g, res.ZZZ, res.ZZ, res.ZZZ, res.ZZ), I);
+    typename F::T v = WP::canon(WP::mul(WP::pick(g, res.X, res.Y, res.X, res.Y), t));
+    uint64_t *o = out + slot * (2 * H + 1);
+    if (g < 2 && w_lane() == 0) store_ref<F>(o + g * H, v);
+    if (threadIdx.x == 0) o[2 * H] = res.inf ? 1u : 0u;
+    return;
+  }
+  // (X ZZZ, Y ZZ, ZZ ZZZ); infinity is (0, 0, 0)
   const typename F::T o =
       WP::canon(WP::mul(WP::pick(g, res.X, res.Y, res.ZZ, res.ZZ), WP::pick(g, res.ZZZ, res.ZZ, res.ZZZ, res.ZZZ)));
   if (g < 3 && w_lane() == 0) {
     typename F::T v = o;
-    const int64_t slot = out_index ? (int64_t)__ldg(out_index + i) : i;
-    store_ref<F>(out_proj + (slot * 3 + g) * (F::LIMBS / 2), v);
+    store_ref<F>(out + (slot * 3 + g) * H, v);
   }
 }
 

@@ -133,8 +133,7 @@ int gm_g2_msm_device_c(gm_stream_t stream, uint32_t gpu_index, G2ProjectivePoint
 /* MSM with an affine result (Montgomery form; infinity flag set for the
  * identity), the device form of point_msm_async<G1Point>/<G2Point>
  * (include/curve.h:238, src/curve.cu:2763), which returns an affine point.
- * Asynchronous: the projective sum is converted to affine by a host
- * function ordered on the stream.  n == 0 writes the point at infinity. */
+ * Asynchronous; the conversion to affine runs on the device. */
 int gm_g1_msm_device_affine(gm_stream_t stream, uint32_t gpu_index, G1Point *d_result, const G1Point *d_points,
                             const uint64_t *d_scalars, int scalar_limbs, int n);
 int gm_g2_msm_device_affine(gm_stream_t stream, uint32_t gpu_index, G2Point *d_result, const G2Point *d_points,

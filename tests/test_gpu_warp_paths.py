@@ -71,3 +71,40 @@ def test_slices_on_warps_and_threads(cuda, group, n, c):
     pts = gm.generator_mul_batch(dev(logs, cuda), group=group)
     want = oracle.generator_multiple(wl.expected_log(sc, logs), group=group)
     assert oracle.same_point(run(pts, sc, group, cuda, c), want)
+
+
+@pytest.mark.parametrize("group", [1, 2])
+@pytest.mark.parametrize("n", [1, 2, 50, 0])
+def test_affine_result(cuda, group, n):
+    """The affine form of the result (an inversion on the device), infinity included."""
+    logs = wl.make_base_logs(max(n, 1), seed=3 + n)[:n]
+    sc = wl.make_scalars(max(n, 1), seed=4 + n)[:n]
+    if n == 2:  # P - P
+        logs[1] = logs[0]
+        sc[0], sc[1] = wl.int_to_limbs(5), wl.int_to_limbs(wl.R_ORDER - 5)
+    words = gm.G1_WORDS if group == 1 else gm.G2_WORDS
+    pts = gm.generator_mul_batch(dev(logs, cuda), group=group) if n else torch.empty((0, words), dtype=torch.int64,
+                                                                                    device=cuda)
+    out = gm.msm_device_affine(pts, dev(sc, cuda), group=group)
+    torch.cuda.synchronize()
+    got = gm.to_numpy_points(out, group)
+    if n in (0, 2):
+        assert bool(got["infinity"][0]) and not got["x"].any() and not got["y"].any()
+    else:
+        assert oracle.same_point(got, oracle.generator_multiple(wl.expected_log(sc, logs), group=group))
+
+
+@pytest.mark.parametrize("group", [1, 2])
+def test_affine_results_of_many_values(cuda, group):
+    """64 one-point MSMs: as many different values through the inversion."""
+    logs = wl.make_base_logs(64, seed=77)
+    pts = gm.generator_mul_batch(dev(logs, cuda), group=group)
+    one = dev(np.array([[3]], dtype=np.uint64), cuda)
+    words = gm.G1_WORDS if group == 1 else gm.G2_WORDS
+    out = torch.zeros((64, words), dtype=torch.int64, device=cuda)
+    for i in range(64):
+        gm.msm_device_affine(pts[i:i + 1], one, group=group, out=out[i])
+    torch.cuda.synchronize()
+    got = gm.to_numpy_points(out, group)
+    for i, t in enumerate(wl.limbs_to_ints(logs)):
+        assert oracle.same_point(got[i:i + 1], oracle.generator_multiple(3 * t, group=group)), i
