@@ -151,7 +151,7 @@ int batch_class_finish(const BatchClassPlan &cp, cudaStream_t s, uint64_t *resul
   rc = reduce_launch<F>(s, cp.rl, cb.buckets, cb.offsets, cp.ws, &src, launches);
   if (rc) return rc;
   // precomputed mode: one window per MSM, so the combination is a conversion
-  k_combine<F><<<(unsigned)cp.count, 32 * COMBINE_WARPS, w_sum_smem<F>(COMBINE_WARPS), s>>>(
+  k_combine<F><<<(unsigned)cp.count, COMBINE_THREADS<F>, combine_smem<F>(), s>>>(
       src, cp.pc_stride ? 1 : cp.dp.W, cp.c, cb.out_index, results, false);
   GM_CHECK_LAUNCH("k_combine");
   (*launches)++;

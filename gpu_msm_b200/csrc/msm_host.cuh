@@ -357,7 +357,7 @@ int msm_run(cudaStream_t s, const MsmLayout<F> &lay, char *ws, const uint4 *base
     handoff->W = W;
     handoff->c = lay.dp.c;
   } else {
-    k_combine<F><<<1, 32 * COMBINE_WARPS, w_sum_smem<F>(COMBINE_WARPS), s>>>(src, W, lay.dp.c, nullptr, out,
+    k_combine<F><<<1, COMBINE_THREADS<F>, combine_smem<F>(), s>>>(src, W, lay.dp.c, nullptr, out,
                                                                                     affine);
     GM_CHECK_LAUNCH("k_combine");
     launches++;

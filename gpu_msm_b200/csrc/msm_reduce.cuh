@@ -21,13 +21,15 @@
 // :2060-2179) with work that stays on the device.
 #pragma once
 #include "msm_kernels.cuh"
-#include "xyzz_warp.cuh"
+#include "xyzz_chain.cuh"
 
 namespace gm {
 
 constexpr int W_THREADS = 128;    // block of the kernels with one warp per work item
 constexpr int SUM_WARPS = 8;      // warps of a block sum
-constexpr int COMBINE_WARPS = 8;  // warps of a window combination
+constexpr int COMBINE_WARPS = 8;  // groups of windows of a window combination
+template <class F>
+constexpr int COMBINE_THREADS = 32 * (COMBINE_WARPS > Chain<F>::WARPS ? COMBINE_WARPS : Chain<F>::WARPS);
 constexpr int W_FILL = 16;        // warps per SM that keep its schedulers busy with dependent point operations
 constexpr int ACC_WARP_MIN = 4;    // entries of a slice on a warp, at least
 constexpr int ACC_WARP_MAX = 16;   // and at most; above W_SLICES slices of these, threads take the slices
@@ -295,40 +297,71 @@ __global__ void __launch_bounds__(32 * SUM_WARPS) k_fixup_long(const uint32_t *_
 }
 
 // ---------------------------------------------------------------------------
-// Window combination on the device, one block of COMBINE_WARPS warps per MSM:
-// result = sum_w 2^(c w) S_w by Horner; homogeneous projective output (u64
-// limbs, Montgomery).  The c (W - 1) doublings of the top window are one
-// serial chain, about 0.9 us each; the additions are kept off it: every warp
-// combines W / COMBINE_WARPS windows, all at once, and warp 0 the warps'
-// sums.  out_index (optional) maps MSM i to its result slot.  affine: an
-// affine point of the reference's layout instead (infinity flag in the word
-// after the coordinates).
+// Window combination on the device, one block per MSM: result = sum_w
+// 2^(c w) S_w by Horner; homogeneous projective output (u64 limbs,
+// Montgomery).  The c (W - 1) doublings of the top window are one serial
+// chain, run by the block's warps together (xyzz_chain.cuh); the additions
+// are kept off it: every warp combines W / COMBINE_WARPS windows, all at once,
+// and the chain takes in the warps' sums.  out_index (optional) maps MSM i to
+// its result slot.  affine: an affine point of the reference's layout instead
+// (infinity flag in the word after the coordinates).
 // ---------------------------------------------------------------------------
 template <class F>
-__global__ void __launch_bounds__(32 * COMBINE_WARPS) k_combine(const xyzz_t<F> *__restrict__ S, int W, int c,
+__global__ void __launch_bounds__(COMBINE_THREADS<F>) k_combine(const xyzz_t<F> *__restrict__ S, int W, int c,
                                                                 const int32_t *__restrict__ out_index,
                                                                 uint64_t *__restrict__ out, bool affine) {
   using WP = WF<F>;
+  constexpr int PT = w_pt_words<F>(), LW = WP::LW;
   w_setup();
   const int64_t i = blockIdx.x;
   const int w = threadIdx.x >> 5;
   const int q = (W + COMBINE_WARPS - 1) / COMBINE_WARPS;
   int32_t *sums = w_smem + w_smem_bytes<F>(COMBINE_WARPS) / 4;
+  int32_t *io = sums + COMBINE_WARPS * PT, *ctl = io + 3 * LW;
+  // the chain works in the scratch of warps 1 and up, which are done by then
+  int32_t *work = w_smem + W_TABLE_WORDS + w_scratch_words<F>();
+  static_assert(chain_words<F>() <= (COMBINE_WARPS - 1) * w_scratch_words<F>(), "chain scratch");
   wpt<F> res = w_inf<F>();
-  for (int j = min(W, (w + 1) * q) - 1; j >= w * q; j--) {
-    if (!res.inf)
-      for (int k = 0; k < c; k++) res = w_dbl<F>(res);
-    res = w_addp<F>(res, w_load_pt<F>(S + i * W + j));
+  if (w < COMBINE_WARPS) {
+    for (int j = min(W, (w + 1) * q) - 1; j >= w * q; j--) {
+      if (!res.inf)
+        for (int k = 0; k < c; k++) res = w_dbl<F>(res);
+      res = w_addp<F>(res, w_load_pt<F>(S + i * W + j));
+    }
+    w_put_pt<F>(sums + w * PT, res);
   }
-  w_put_pt<F>(sums + w * w_pt_words<F>(), res);
   __syncthreads();
-  if (w > 0) return;
-  res = w_get_pt<F>(sums + (COMBINE_WARPS - 1) * w_pt_words<F>());
-  for (int j = COMBINE_WARPS - 2; j >= 0; j--) {
-    if (!res.inf)
-      for (int k = 0; k < c * q; k++) res = w_dbl<F>(res);
-    res = w_addp<F>(res, w_get_pt<F>(sums + j * w_pt_words<F>()));
+  if (w >= Chain<F>::WARPS) return;
+  int top = (W + q - 1) / q - 1;
+  while (top > 0 && sums[top * PT + 4 * LW] != 0) top--;  // windows at infinity
+  res = w_get_pt<F>(sums + top * PT);
+  for (int j = top - 1; j >= 0; j--) {
+    if (w == 0) {
+      if (threadIdx.x == 0) ctl[0] = res.inf ? 1 : 0;
+      WP::put(io, res.X);
+      WP::put(io + LW, res.Y);
+      WP::put(io + 2 * LW, WP::one());
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * Chain<F>::WARPS) : "memory");
+    if (ctl[0] == 0) chain_dbl<F>(c * q, io, work);
+    if (w == 0) {
+      if (!res.inf) {
+        const typename WP::E L = WP::get(io + 2 * LW);
+        res.X = WP::get(io);
+        res.Y = WP::get(io + LW);
+        const int g = w_group();
+        const typename WP::E t = WP::mul(WP::pick(g, L, res.ZZZ, L, L), L);
+        const typename WP::E LL = WP::from(t, 0);
+        const typename WP::E z = WP::mul(WP::pick(g, res.ZZ, WP::from(t, 1), LL, LL), LL);
+        res.ZZ = WP::from(z, 0);
+        res.ZZZ = WP::from(z, 1);
+        if (WP::is_zero(L)) res = w_inf<F>();  // a point of order two was doubled
+      }
+      res = w_addp<F>(res, w_get_pt<F>(sums + j * PT));
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * Chain<F>::WARPS) : "memory");
   }
+  if (w > 0) return;
   constexpr int H = F::LIMBS / 2;
   const int g = w_group();
   const int64_t slot = out_index ? (int64_t)__ldg(out_index + i) : i;
@@ -350,6 +383,11 @@ __global__ void __launch_bounds__(32 * COMBINE_WARPS) k_combine(const xyzz_t<F> 
     typename F::T v = o;
     store_ref<F>(out + (slot * 3 + g) * H, v);
   }
+}
+
+template <class F>
+constexpr int combine_smem() {
+  return w_sum_smem<F>(COMBINE_WARPS) + 4 * (3 * WF<F>::LW + 4);
 }
 
 // ---------------------------------------------------------------------------
