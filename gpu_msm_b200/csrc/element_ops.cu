@@ -65,20 +65,6 @@ GM_DEVI fp_t one_std() {
 // Montgomery-form Fp with every product out of line: one copy of the
 // ~900-instruction product per kernel instead of one per call site keeps
 // these single-thread kernels small and quick to compile.
-__device__ __noinline__ fp_t f1_inv(fp_t a) {
-  // a^(p-2), left-to-right square-and-multiply; 0 -> 0 (src/fp.cu:545)
-  fp_t acc;
-#pragma unroll
-  for (int i = 0; i < NL; i++) acc.v[i] = gm::FpConst::ONE(i);
-  for (int w = NL - 1; w >= 0; w--) {
-    const uint32_t e = (w == 0) ? gm::FpConst::P(0) - 2u : gm::FpConst::P(w);
-    for (int b = 31; b >= 0; b--) {
-      acc = gm::fp_sqr_call(acc);
-      if ((e >> b) & 1u) acc = gm::fp_mul_call(acc, a);
-    }
-  }
-  return acc;
-}
 struct F1 : gm::FpOut {
   GM_DEVI static fp_t to_mont(const fp_t &a) { return mul(a, r2_const()); }
   GM_DEVI static fp_t from_mont(const fp_t &a) {
@@ -86,7 +72,6 @@ struct F1 : gm::FpOut {
     o.v[0] = 1;
     return mul(a, o);
   }
-  GM_DEVI static fp_t inv(const fp_t &a) { return f1_inv(a); }
 };
 using F2 = gm::Fp2T<F1>;  // Montgomery-form Fp2 over F1
 

@@ -10,8 +10,13 @@
 // what is left, which is one point of most buckets and the rest of the few
 // that are much larger, so those need no rule of their own here.
 //
-// Bound: the multiplier, as for k_accumulate (a round reads two records twice
-// and writes one and a prefix product, 600 bytes an addition, about 2 TB/s).
+// Bound: the multiplier, as for k_accumulate (a round moves 640 bytes an
+// addition, 1.5 TB/s).  B200, G1 2^20 (19.5 M entries, 28 to a bucket): 0.42 ns
+// an addition in the first rounds against 0.55 ns in k_accumulate; accumulation
+// in all 11.1 -> 8.8 ms, G2 2^18 8.7 -> 7.0 ms.  Three blocks of 128 threads
+// per SM (G1): two measured 9.14 ms against 8.79 for six rounds, four 9.00 (the
+// code of product, square, inversion and loops then outgrows the instruction
+// cache).
 //
 // The points of a round lie in bucket order: round r's offsets are the prefix
 // sums of ceil(s / 2^r), all computed at once from the sorted entries'
@@ -21,7 +26,6 @@
 // the rounds alternate between stay within AFF_SCRATCH bytes.
 #pragma once
 #include <algorithm>
-#include <cmath>
 #include <vector>
 
 #include "msm_kernels.cuh"
@@ -29,11 +33,14 @@
 namespace gm {
 
 constexpr int AFF_THREADS = 128;
-constexpr int AFF_BATCH = 32;       // additions that share an inversion
+constexpr int AFF_BATCH = 64;       // additions that share an inversion, at most
 constexpr int AFF_MIN = 16;         // outputs of a thread, at least (a shorter run spends more on its inversion)
 constexpr int AFF_MAX_ROUNDS = 8;
-constexpr int64_t AFF_MIN_ENTRIES = 1500000;
-constexpr int AFF_MIN_AVG = 6;
+// Outputs per thread of the last round, at least.  Measured with 10 / 16 / 24
+// / 40: G1 2^20 11.52 / 11.41 / 11.38 / 11.40 ms, G1 2^18 4.23 / 4.18 / 4.18 /
+// 4.25, G1 200000 3.41 / 3.34 / 3.46 / 3.46, G2 130000 6.18 / 6.13 / 6.48 / 6.47,
+// G2 65536 4.33 / 4.27 / 4.60 / 4.60 (without rounds: 13.66, 4.56, 3.77, 7.23, 4.60).
+constexpr int AFF_LAST = 16;
 constexpr size_t AFF_SCRATCH = size_t(3) << 30;
 template <class F>
 constexpr int AFF_BLOCKS = sizeof(typename F::T) == sizeof(fp_t) ? 3 : 2;  // resident blocks per SM
@@ -44,7 +51,7 @@ template <class F>
 struct AffPolicy;
 template <>
 struct AffPolicy<Fp> {
-  using type = FpOutMulOnly;
+  using type = FpOut;
 };
 template <>
 struct AffPolicy<Fp2> {
@@ -198,17 +205,15 @@ struct AffWalk {
   }
 };
 
-// Shared-memory stage of one thread: the records of the next pair arrive with
-// cp.async while the current one is worked on.  [slot][chunk][thread] uint4.
-// G1 stages x and y of both points and the prefix product; G2 only the x's
-// and the prefix (two blocks' stages would not fit an SM with the y's too).
+// Shared-memory stage of one thread ([chunk][thread] uint4): the two points
+// of a pair and its prefix product, brought in with cp.async while a product
+// of the same or the previous addition runs, so one slot is enough.
 template <class F>
 struct AffStage {
-  static constexpr bool YS = sizeof(typename F::T) == sizeof(fp_t);
-  static constexpr int XC = (F::LIMBS + 3) / 4;          // chunks of x (Fp: and the first 2 words of y)
-  static constexpr int RC = YS ? F::LIMBS / 2 : XC;      // chunks of a point
-  static constexpr int CH = 2 * RC + XC;                 // P, Q, prefix
-  static constexpr int BYTES = 2 * CH * AFF_THREADS * 16;
+  static constexpr int XC = (F::LIMBS + 3) / 4;  // chunks of an element (Fp: and the first 2 words of y)
+  static constexpr int RC = F::LIMBS / 2;        // chunks of a point
+  static constexpr int CH = 2 * RC + XC;         // P, Q, prefix
+  static constexpr int BYTES = CH * AFF_THREADS * 16;
 };
 
 template <class F>
@@ -252,7 +257,8 @@ __global__ void __launch_bounds__(AFF_THREADS, AFF_BLOCKS<F>)
   using S = AffStage<F>;
   constexpr int L = F::LIMBS, U4 = Rec<F>::U4;
   extern __shared__ uint4 stage_mem[];
-  auto stage = reinterpret_cast<uint4(*)[S::CH][AFF_THREADS]>(stage_mem);
+  auto stage = reinterpret_cast<uint4(*)[AFF_THREADS]>(stage_mem);
+  const uint4(*const P)[AFF_THREADS] = stage, (*const Q)[AFF_THREADS] = stage + S::RC, (*const R)[AFF_THREADS] = stage + 2 * S::RC;
   const int tid = threadIdx.x;
   const uint32_t o0 = __ldg(off_out + k0), o1 = __ldg(off_out + k1);
   const uint32_t nthr = gridDim.x * blockDim.x, t = blockIdx.x * blockDim.x + tid;
@@ -271,42 +277,37 @@ __global__ void __launch_bounds__(AFF_THREADS, AFF_BLOCKS<F>)
     load_coord<F>(y, rec(e), true);
     return FIRST && (e & 1u) ? F::neg(y) : y;
   };
-  auto copy = [&](int slot, int c, const uint4 *src, int n) {
-    for (int q = 0; q < n; q++) cp_async16(&stage[slot][c + q][tid], src + q);
-  };
   auto pre = [&](int i, int q) -> uint4 * { return prefix + ((size_t)i * S::XC + q) * nthr + t; };
 
-  for (uint32_t s0 = (uint32_t)start64; s0 < end; s0 += AFF_BATCH) {
-    const int cnt = (int)min(end - s0, (uint32_t)AFF_BATCH);
-    uint32_t m_mul = 0, m_dbl = 0, m_b = 0, m_inf = 0;  // additions, doublings among them, copies of q, infinity
+  // equal batches
+  const uint32_t nbatch = (end - (uint32_t)start64 + AFF_BATCH - 1) / AFF_BATCH;
+  const uint32_t bsize = (end - (uint32_t)start64 + nbatch - 1) / nbatch;
+  for (uint32_t s0 = (uint32_t)start64; s0 < end; s0 += bsize) {
+    const int cnt = (int)min(end - s0, bsize);
+    uint64_t m_mul = 0, m_dbl = 0, m_b = 0, m_inf = 0;  // additions, doublings among them, copies of q, infinity
     T run;
-    AffPair c0, c1 = walk.forward(s0), c2 = cnt > 1 ? walk.forward(s0 + 1) : c1;
-    int slot = 0;
-    auto stage_x = [&](int sl, const AffPair &c) {
+    AffPair c0, c1 = walk.forward(s0);
+    auto stage_x = [&](const AffPair &c) {
       if (c.pair) {
 #pragma unroll
         for (int q = 0; q < S::XC; q++) {
-          cp_async16(&stage[sl][q][tid], rec(c.p) + q);
-          cp_async16(&stage[sl][S::RC + q][tid], rec(c.q) + q);
+          cp_async16(&stage[q][tid], rec(c.p) + q);
+          cp_async16(&stage[S::RC + q][tid], rec(c.q) + q);
         }
       }
       cp_async_commit();
     };
-    stage_x(0, c1);
+    stage_x(c1);
 #pragma unroll 1
-    for (int i = 0; i < cnt; i++, slot ^= 1) {
+    for (int i = 0; i < cnt; i++) {
       c0 = c1;
-      c1 = c2;
-      if (i + 1 < cnt)
-        stage_x(slot ^ 1, c1);
-      else
-        cp_async_commit();
-      if (i + 2 < cnt) c2 = walk.forward(s0 + i + 2);
-      cp_async_wait_prev();
-      if (!c0.pair) continue;  // the odd point out
+      if (i + 1 < cnt) c1 = walk.forward(s0 + i + 1);
+      cp_async_wait<0>();
+      const T x1 = stage_get<F>(P, tid, 0);
+      T d = stage_get<F>(Q, tid, 0);
+      if (i + 1 < cnt) stage_x(c1);  // the next x's arrive during this product
+      if (!c0.pair) continue;        // the odd point out
       bool add = true;
-      const T x1 = stage_get<F>(&stage[slot][0], tid, 0);
-      T d = stage_get<F>(&stage[slot][S::RC], tid, 0);
       const bool z1 = F::is_zero_raw(x1), z2 = F::is_zero_raw(d);
       d = F::sub(d, x1);
       const bool e = F::is_zero_raw(d);
@@ -314,14 +315,14 @@ __global__ void __launch_bounds__(AFF_THREADS, AFF_BLOCKS<F>)
         const T y1 = coord_y(c0.p), y2 = coord_y(c0.q);
         const bool i1 = z1 && F::is_zero_raw(y1), i2 = z2 && F::is_zero_raw(y2);
         if (i1 || i2) {
-          if (i1) m_b |= 1u << i;  // infinity + q, also when q is infinity
+          if (i1) m_b |= 1ull << i;  // infinity + q, also when q is infinity
           add = false;
         } else if (e) {
           if (F::eq(y1, y2) && !F::is_zero_raw(y1)) {
             d = F::dbl(y1);
-            m_dbl |= 1u << i;
+            m_dbl |= 1ull << i;
           } else {
-            m_inf |= 1u << i;
+            m_inf |= 1ull << i;
             add = false;
           }
         }
@@ -341,7 +342,7 @@ __global__ void __launch_bounds__(AFF_THREADS, AFF_BLOCKS<F>)
         } else {
           run = d;
         }
-        m_mul |= 1u << i;
+        m_mul |= 1ull << i;
       }
     }
     T inv;
@@ -349,54 +350,46 @@ __global__ void __launch_bounds__(AFF_THREADS, AFF_BLOCKS<F>)
     __threadfence();  // this thread's prefix products, which come back through cp.async
 
     const AffWalk<FIRST> ahead = walk;  // where the next batch goes on
-    auto stage_all = [&](int sl, int i, const AffPair &c) {
-      const uint32_t bit = 1u << i;
-      if (m_mul & bit) {
-        const uint4 *p = rec(c.p), *q = rec(c.q);
+    auto stage_prefix = [&](int i) {
+      if (i >= 0 && (m_mul >> i & 1) && (m_mul & ((1ull << i) - 1))) {
 #pragma unroll
-        for (int w = 0; w < S::RC; w++) {
-          cp_async16(&stage[sl][w][tid], p + w);
-          cp_async16(&stage[sl][S::RC + w][tid], q + w);
-        }
-        if (m_mul & (bit - 1)) {
-#pragma unroll
-          for (int w = 0; w < S::XC; w++) cp_async16(&stage[sl][2 * S::RC + w][tid], pre(i, w));
-        }
+        for (int w = 0; w < S::XC; w++) cp_async16(&stage[2 * S::RC + w][tid], pre(i, w));
       }
       cp_async_commit();
     };
+    stage_prefix(cnt - 1);
     c1 = walk.backward(s0 + cnt - 1);
-    c2 = cnt > 1 ? walk.backward(s0 + cnt - 2) : c1;
-    slot = 0;
-    stage_all(0, cnt - 1, c1);
 #pragma unroll 1
-    for (int i = cnt - 1; i >= 0; i--, slot ^= 1) {
-      const uint32_t bit = 1u << i;
+    for (int i = cnt - 1; i >= 0; i--) {
+      const uint64_t bit = 1ull << i;
       c0 = c1;
-      c1 = c2;
-      if (i > 0)
-        stage_all(slot ^ 1, i - 1, c1);
-      else
-        cp_async_commit();
-      if (i > 1) c2 = walk.backward(s0 + i - 2);
-      cp_async_wait_prev();
-      uint4 *dst = out + (size_t)(s0 + i) * U4;
-      const uint4(*P)[AFF_THREADS] = &stage[slot][0];
-      const uint4(*Q)[AFF_THREADS] = &stage[slot][S::RC];
-      auto y_of = [&](const uint4(*c)[AFF_THREADS], uint32_t e) -> T {
-        if constexpr (S::YS) {
-          const T y = stage_get<F>(c, tid, L);
-          return FIRST && (e & 1u) ? F::neg(y) : y;
-        } else {
-          return coord_y(e);
+      if (m_mul & bit) {
+        const uint4 *p = rec(c0.p), *q = rec(c0.q);
+#pragma unroll
+        for (int w = 0; w < S::RC; w++) {
+          cp_async16(&stage[w][tid], p + w);
+          cp_async16(&stage[S::RC + w][tid], q + w);
         }
+      }
+      cp_async_commit();
+      if (i > 0) c1 = walk.backward(s0 + i - 1);
+      uint4 *dst = out + (size_t)(s0 + i) * U4;
+      auto y_of = [&](const uint4(*c)[AFF_THREADS], uint32_t e) -> T {
+        const T y = stage_get<F>(c, tid, L);
+        return FIRST && (e & 1u) ? F::neg(y) : y;
       };
       if (m_mul & bit) {
         const bool dbl = (m_dbl & bit) != 0;
         T lam = inv;
+        cp_async_wait<1>();  // the prefix product
         if (m_mul & (bit - 1)) {  // not the batch's first addition
-          lam = A::mul(stage_get<F>(&stage[slot][2 * S::RC], tid, 0), inv);
+          lam = stage_get<F>(R, tid, 0);
+          stage_prefix(i - 1);
+          lam = A::mul(lam, inv);
+          cp_async_wait<1>();  // the points
           inv = A::mul(inv, dbl ? F::dbl(y_of(P, c0.p)) : F::sub(stage_get<F>(Q, tid, 0), stage_get<F>(P, tid, 0)));
+        } else {
+          cp_async_wait<0>();
         }
         T num;
         if (dbl) {
@@ -415,7 +408,9 @@ __global__ void __launch_bounds__(AFF_THREADS, AFF_BLOCKS<F>)
       } else if (m_inf & bit) {
         T z = F::zero();
         store_point<F>(dst, z, z);
+        stage_prefix(i - 1);
       } else {
+        stage_prefix(i - 1);
         const uint32_t e = (m_b & bit) ? c0.q : c0.p;
         T x, y = coord_y(e);
         load_coord<F>(x, rec(e), false);
@@ -423,8 +418,7 @@ __global__ void __launch_bounds__(AFF_THREADS, AFF_BLOCKS<F>)
       }
     }
     walk = ahead;
-    // the next batch reuses this thread's stage
-    asm volatile("cp.async.wait_all;" ::: "memory");
+    cp_async_wait<0>();  // the next batch reuses this thread's stage
   }
 }
 
@@ -438,34 +432,37 @@ struct AffLayout {
     int64_t k0, k1;
   };
   std::vector<Chunk> chunks;
-  // in the accumulation's workspace: offsets of every round, block sums, the points left over
-  size_t o_off = 0, o_bsum = 0, o_fin = 0;
+  // own memory: offsets of every round, block sums, the points left over
+  size_t bytes = 0, o_off = 0, o_bsum = 0, o_fin = 0;
   // scratch of the rounds (accumulations that run one after another can share it)
   size_t scratch = 0, s_buf1 = 0, s_prefix = 0;
   unsigned grid = 0;
 
-  const uint32_t *final_offsets(const char *ws) const {
-    return (const uint32_t *)(ws + o_off) + (int64_t)(rounds - 1) * (K + 1);
+  // what the rounds leave in the own memory m: points in bucket order, and their offsets
+  const uint32_t *final_offsets(const char *m) const {
+    return (const uint32_t *)(m + o_off) + (int64_t)(rounds - 1) * (K + 1);
   }
+  const uint4 *final_points(const char *m) const { return (const uint4 *)(m + o_fin); }
 
   // sizes: points of the MSMs; each has `groups` key groups (windows, or 1
   // over a fixed-base table) of B keys, every group at most per_point entries
   // per point.  K keys in all.
   //
-  // Rounds pay where a thread's run of pairs shares its inversion and buckets
-  // hold several points: at least AFF_MIN_ENTRIES entries and AFF_MIN_AVG per
-  // bucket.  Their number brings a bucket of avg + 4 sqrt(avg) points to one.
+  // A round pays while its threads have enough outputs to share an inversion
+  // and buckets still hold two points or more.
   template <class F, class Carver>
-  void plan(const int64_t *sizes, int count, int groups, int per_point, int B, int sms, Carver &cv) {
+  void plan(const int64_t *sizes, int count, int groups, int per_point, int B, int sms) {
+    Carver cv;
     int64_t E = 0;
     for (int i = 0; i < count; i++) E += sizes[i] * per_point * groups;
     K = (int64_t)count * groups * B;
     const double avg = (double)E / (double)K;
-    if (E < AFF_MIN_ENTRIES || avg < AFF_MIN_AVG) return;
     constexpr size_t REC = Rec<F>::U4 * sizeof(uint4);
-    const double most = avg + 4.0 * std::sqrt(avg);
-    int R = 1;
-    while (R < AFF_MAX_ROUNDS && (double)(1 << R) < most) R++;
+    grid = (unsigned)(sms * AFF_BLOCKS<F>);
+    const int64_t threads = (int64_t)grid * AFF_THREADS;
+    int R = 0;
+    while (R < AFF_MAX_ROUNDS && (E >> (R + 1)) >= AFF_LAST * threads && (2 << R) <= avg) R++;
+    if (R == 0) return;
     // outputs of a chunk of e entries and k keys after r + 1 rounds
     auto outputs = [](int64_t e, int64_t k, int r) {
       return std::min(e, ((e + k * ((int64_t(2) << r) - 1)) >> (r + 1)) + 1);
@@ -497,7 +494,7 @@ struct AffLayout {
     o_off = cv.template take<uint32_t>((size_t)(R * (K + 1)));
     o_bsum = cv.template take<uint32_t>((size_t)(R * nb));
     o_fin = cv.template take<uint4>((size_t)outputs(E, K, R - 1) * Rec<F>::U4);
-    grid = (unsigned)(sms * AFF_BLOCKS<F>);
+    bytes = cv.off;
     auto up = [](size_t x) { return (x + 255) / 256 * 256; };
     s_buf1 = up((size_t)b0 * REC);
     s_prefix = s_buf1 + (R > 1 ? up((size_t)b1 * REC) : 0);
@@ -505,10 +502,9 @@ struct AffLayout {
   }
 };
 
-// Enqueues the rounds on s.  Afterwards the points left are ws + o_fin, in
-// bucket order under final_offsets(ws).
+// Enqueues the rounds on s, in the layout's own memory m and the scratch.
 template <class F>
-cudaError_t aff_launch(cudaStream_t s, const AffLayout &lay, char *ws, char *scratch, const uint4 *bases,
+cudaError_t aff_launch(cudaStream_t s, const AffLayout &lay, char *m, char *scratch, const uint4 *bases,
                        const uint32_t *entries, const uint32_t *off0, int *launches) {
   const int R = lay.rounds;
   const int64_t K = lay.K;
@@ -517,8 +513,8 @@ cudaError_t aff_launch(cudaStream_t s, const AffLayout &lay, char *ws, char *scr
     if (e != cudaSuccess) return e;
   }
   const unsigned nb = (unsigned)((K + SCAN_TILE - 1) / SCAN_TILE);
-  auto *off = (uint32_t *)(ws + lay.o_off);
-  auto *bsum = (uint32_t *)(ws + lay.o_bsum);
+  auto *off = (uint32_t *)(m + lay.o_off);
+  auto *bsum = (uint32_t *)(m + lay.o_bsum);
   k_aff_blocksum<<<dim3(nb, R), SCAN_THREADS, 0, s>>>(off0, K, bsum);
   k_aff_top<<<R, SCAN_THREADS, 0, s>>>(bsum, (int)nb);
   k_aff_offsets<<<dim3(nb, R), SCAN_THREADS, 0, s>>>(off0, K, bsum, off, K + 1);
@@ -528,7 +524,7 @@ cudaError_t aff_launch(cudaStream_t s, const AffLayout &lay, char *ws, char *scr
   for (const auto &c : lay.chunks) {
     for (int r = 0; r < R; r++) {
       const uint32_t *off_out = off + (int64_t)r * (K + 1);
-      uint4 *out = r == R - 1 ? (uint4 *)(ws + lay.o_fin) : buf[r & 1];
+      uint4 *out = r == R - 1 ? (uint4 *)(m + lay.o_fin) : buf[r & 1];
       if (r == 0)
         k_affine_round<F, true><<<lay.grid, AFF_THREADS, AffStage<F>::BYTES, s>>>(bases, entries, off0, off_out, c.k0, c.k1, out,
                                                                  r < R - 1, prefix);

@@ -58,6 +58,7 @@ namespace {
 void free_plan(gm_batch_plan *p) {
   for (auto &cp : p->plan.classes) {
     if (cp.ws) cudaFree(cp.ws);
+    if (cp.aff_ws) cudaFree(cp.aff_ws);
     if (cp.desc) cudaFree(cp.desc);
     if (cp.stream) cudaStreamDestroy(cp.stream);
     if (cp.done) cudaEventDestroy(cp.done);
@@ -66,8 +67,34 @@ void free_plan(gm_batch_plan *p) {
   if (p->plan.fork) cudaEventDestroy(p->plan.fork);
   if (p->plan.acc_done) cudaEventDestroy(p->plan.acc_done);
   if (p->plan.acc_desc) cudaFree(p->plan.acc_desc);
+  if (p->plan.aff_scratch) cudaFree(p->plan.aff_scratch);
   if (p->plan.queue_ctr) cudaFree(p->plan.queue_ctr);
   delete p;
+}
+
+// The memory of the plan's affine rounds; the plan runs without them where the
+// device does not have it four times over.
+void plan_rounds(gm::BatchPlan &plan) {
+  const size_t scratch = plan.aff_scratch_bytes();
+  if (scratch == 0) return;
+  size_t need = scratch, free_bytes = 0, all = 0;
+  for (const auto &cp : plan.classes) need += cp.al.bytes;
+  if (cudaMemGetInfo(&free_bytes, &all) != cudaSuccess || free_bytes < 4 * need ||
+      cudaMalloc(&plan.aff_scratch, scratch) != cudaSuccess) {
+    cudaGetLastError();
+    plan.aff_scratch = nullptr;
+    return;
+  }
+  plan.bytes += scratch;
+  for (auto &cp : plan.classes) {
+    if (cp.al.rounds == 0) continue;
+    if (cudaMalloc(&cp.aff_ws, cp.al.bytes) != cudaSuccess) {
+      cudaGetLastError();
+      cp.aff_ws = nullptr;
+      continue;
+    }
+    plan.bytes += cp.al.bytes;
+  }
 }
 
 // Validates the batch, groups MSMs by window width and computes each class's
@@ -143,6 +170,7 @@ int build_classes(const gm_bases *b, int scalar_limbs, int count, const int64_t 
     }
     const int64_t tp = (int64_t)gm::SA_THREADS * cp.sort_ppt;
     for (int i : kv.second) {
+      cp.sizes.push_back(sizes[i]);
       cp.P += sizes[i];
       cp.tilesA += (sizes[i] + tp - 1) / tp;
     }
@@ -352,6 +380,7 @@ int gm_batch_plan_create_tuned(const gm_bases *b, int scalar_limbs, int count, c
     }
     plan.bytes += cp.ws_bytes + desc_bytes;
   }
+  plan_rounds(plan);
   cudaError_t e = cudaEventCreateWithFlags(&plan.fork, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&plan.acc_done, cudaEventDisableTiming);
   // descriptors of the queued accumulation (used when the plan's mode is set)
@@ -413,6 +442,16 @@ static int batch_run_once(gm_stream_t stream, const gm_bases *b, int scalar_limb
     off_ws[k] = total;
     total += (plan.classes[k].ws_bytes + 255) / 256 * 256;
   }
+  // the affine rounds' memory behind it, where there is room for it
+  std::vector<size_t> off_aff(plan.classes.size());
+  size_t with_rounds = total;
+  for (size_t k = 0; k < plan.classes.size(); k++) {
+    off_aff[k] = with_rounds;
+    with_rounds += (plan.classes[k].al.bytes + 255) / 256 * 256;
+  }
+  const size_t off_scratch = with_rounds;
+  with_rounds += plan.aff_scratch_bytes();
+  bool rounds = with_rounds > total;
   char *mem = nullptr;
   if (ws) {
     if (total > ws_bytes || (size_t)transient_bytes(plan, d64, idx) > ws_bytes ||
@@ -421,10 +460,17 @@ static int batch_run_once(gm_stream_t stream, const gm_bases *b, int scalar_limb
       return gm::GM_ERR_ARG;
     }
     mem = static_cast<char *>(ws);
+    rounds = rounds && with_rounds <= ws_bytes;
   } else {
-    rc = gm::pool_alloc(plan.dev, s, total, (void **)&mem);
+    rc = rounds ? gm::pool_alloc(plan.dev, s, with_rounds, (void **)&mem) : gm::GM_ERR_ALLOC;
+    if (rc) {
+      if (rounds) cudaGetLastError();  // the failed allocation
+      rounds = false;
+      rc = gm::pool_alloc(plan.dev, s, total, (void **)&mem);
+    }
     if (rc) return rc;
   }
+  if (rounds) plan.aff_scratch = mem + off_scratch;
   // descriptors go through one pinned slot (an asynchronous copy from pageable
   // memory would first wait for the stream), released in stream order
   void *slot = nullptr;
@@ -433,6 +479,7 @@ static int batch_run_once(gm_stream_t stream, const gm_bases *b, int scalar_limb
     gm::BatchClassPlan &cp = plan.classes[k];
     cp.desc = mem + off_desc[k];
     cp.ws = mem + off_ws[k];
+    if (rounds) cp.aff_ws = mem + off_aff[k];
     const size_t n64 = d64[k].size() * sizeof(int64_t), n32 = idx[k].size() * sizeof(int32_t);
     cudaError_t e;
     if (pinned) {

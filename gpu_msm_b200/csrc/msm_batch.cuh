@@ -20,6 +20,7 @@ struct BatchClassPlan {
   int c = 0;
   DigitParams dp{};
   int count = 0;        // MSMs in this class
+  std::vector<int64_t> sizes;  // their points
   int64_t P = 0;        // points in this class
   int64_t K = 0, nthreads = 0;
   bool warp_acc = false;  // accumulation slices on warps (then outside the queued launch)
@@ -36,6 +37,9 @@ struct BatchClassPlan {
          o_err = 0;
   size_t ws_bytes = 0;
   char *ws = nullptr;       // workspace (owned)
+  // rounds of affine additions; used where aff_ws and the plan's aff_scratch are there
+  AffLayout al;
+  char *aff_ws = nullptr;   // al.bytes (owned)
   // descriptors (owned): int64 point_start[count+1] | base_off[count] |
   // sc_off[count], then int32 out_index[count] | tile_first[count+1]
   char *desc = nullptr;
@@ -51,6 +55,13 @@ struct BatchPlan {
   std::vector<BatchClassPlan> classes;
   cudaEvent_t fork = nullptr;
   size_t bytes = 0;
+  char *aff_scratch = nullptr;  // scratch of the affine rounds, which run class after class (owned)
+  size_t aff_scratch_bytes() const {
+    size_t b = 0;
+    for (const auto &cp : classes) b = std::max(b, cp.al.scratch);
+    return b;
+  }
+  bool rounds(const BatchClassPlan &cp) const { return cp.al.rounds > 0 && cp.aff_ws && aff_scratch; }
   // Accumulation mode of plans: true (default) = every class's accumulation
   // in one persistent launch over a device work queue (k_accumulate_queue)
   // between the classes' sorts and their fix-ups; false = one pipeline per
@@ -97,17 +108,24 @@ void batch_class_layout(BatchClassPlan &cp, int limbs, int sms, int dev) {
   cp.o_longq = cv.take<int32_t>((size_t)(1 + cp.long_cap));
   cp.o_err = cv.take<uint32_t>(4);
   cp.ws_bytes = cv.off;
+  cp.al = AffLayout();
+  if (!cp.warp_acc)
+    cp.al.plan<F, Carve>(cp.sizes.data(), cp.count, cp.pc_stride ? 1 : cp.dp.W, cp.pc_stride ? cp.dp.W : 1, cp.dp.B,
+                         sms);
 }
 
 // Pointers into one class's workspace.
 template <class F>
 struct ClassBufs {
   uint32_t *offsets, *entries, *err;
+  // what is accumulated: the sorted entries over the bases, or what the affine rounds leave
+  const uint4 *acc_bases;
+  const uint32_t *acc_entries, *acc_offsets;
   int32_t *hk, *tk, *long_q;
   xyzz_t<F> *buckets, *head, *tail;
   SortDesc sd;
   const int32_t *out_index;
-  ClassBufs(const BatchClassPlan &cp) {
+  ClassBufs(const BatchPlan &plan, const BatchClassPlan &cp, bool rounds) {
     char *ws = cp.ws;
     offsets = (uint32_t *)(ws + cp.o_offsets);
     entries = (uint32_t *)(ws + cp.o_entries);
@@ -118,6 +136,14 @@ struct ClassBufs {
     tk = (int32_t *)(ws + cp.o_tk);
     err = (uint32_t *)(ws + cp.o_err);
     long_q = (int32_t *)(ws + cp.o_longq);
+    acc_bases = cp.pc_table ? cp.pc_table : plan.bases;
+    acc_entries = entries;
+    acc_offsets = offsets;
+    if (rounds) {
+      acc_bases = cp.al.final_points(cp.aff_ws);
+      acc_entries = nullptr;
+      acc_offsets = cp.al.final_offsets(cp.aff_ws);
+    }
     sd.point_start = (const int64_t *)cp.desc;
     sd.base_off = sd.point_start + cp.count + 1;
     sd.sc_off = sd.base_off + cp.count;
@@ -130,8 +156,9 @@ struct ClassBufs {
 
 // One class, first part: flags cleared, entries sorted.
 template <class F>
-int batch_class_sort(const BatchClassPlan &cp, cudaStream_t s, const uint64_t *scalars, int *launches) {
-  ClassBufs<F> cb(cp);
+int batch_class_sort(const BatchPlan &plan, const BatchClassPlan &cp, cudaStream_t s, const uint64_t *scalars,
+                     int *launches) {
+  ClassBufs<F> cb(plan, cp, false);
   GM_CHECK(cudaMemsetAsync(cb.err, 0, sizeof(uint32_t), s));
   GM_CHECK(cudaMemsetAsync(cb.long_q, 0, sizeof(int32_t), s));
   const cudaError_t e = sort_launch(s, cp.sl, cp.ws, scalars, cb.sd, cp.K, cb.offsets, cb.entries, launches);
@@ -142,13 +169,14 @@ int batch_class_sort(const BatchClassPlan &cp, cudaStream_t s, const uint64_t *s
 // One class, last part (after its accumulation): fix-up, reduction, and the
 // window combination into the class's result slots.
 template <class F>
-int batch_class_finish(const BatchClassPlan &cp, cudaStream_t s, uint64_t *results, int *launches) {
-  ClassBufs<F> cb(cp);
-  int rc = fixup_launch<F>(s, cb.offsets, cp.K, cp.nthreads, cb.buckets, cb.head, cb.tail, cb.hk, cb.tk, cb.err,
+int batch_class_finish(const BatchPlan &plan, const BatchClassPlan &cp, cudaStream_t s, bool rounds, uint64_t *results,
+                       int *launches) {
+  ClassBufs<F> cb(plan, cp, rounds);
+  int rc = fixup_launch<F>(s, cb.acc_offsets, cp.K, cp.nthreads, cb.buckets, cb.head, cb.tail, cb.hk, cb.tk, cb.err,
                            cb.long_q, cp.long_cap, launches);
   if (rc) return rc;
   const xyzz_t<F> *src = nullptr;
-  rc = reduce_launch<F>(s, cp.rl, cb.buckets, cb.offsets, cp.ws, &src, launches);
+  rc = reduce_launch<F>(s, cp.rl, cb.buckets, cb.acc_offsets, cp.ws, &src, launches);
   if (rc) return rc;
   // precomputed mode: one window per MSM, so the combination is a conversion
   k_combine<F><<<(unsigned)cp.count, COMBINE_THREADS<F>, combine_smem<F>(), s>>>(
@@ -158,27 +186,41 @@ int batch_class_finish(const BatchClassPlan &cp, cudaStream_t s, uint64_t *resul
   return GM_OK;
 }
 
+// One class, the affine rounds over its sorted entries.
 template <class F>
-int batch_class_accumulate(const BatchPlan &plan, const BatchClassPlan &cp, cudaStream_t s, int *launches) {
-  ClassBufs<F> cb(cp);
-  acc_launch<F>(cp.warp_acc, s, cp.pc_table ? cp.pc_table : plan.bases, cb.entries, cb.offsets, cp.K, cp.nthreads,
-                cb.buckets, cb.head, cb.tail, cb.hk, cb.tk);
+int batch_class_rounds(const BatchPlan &plan, const BatchClassPlan &cp, cudaStream_t s, int *launches) {
+  ClassBufs<F> cb(plan, cp, false);
+  const cudaError_t e = aff_launch<F>(s, cp.al, cp.aff_ws, plan.aff_scratch, cb.acc_bases, cb.acc_entries,
+                                      cb.acc_offsets, launches);
+  return e == cudaSuccess ? GM_OK : record_error(e, "k_affine_round");
+}
+
+template <class F>
+int batch_class_accumulate(const BatchPlan &plan, const BatchClassPlan &cp, cudaStream_t s, bool rounds,
+                           int *launches) {
+  ClassBufs<F> cb(plan, cp, rounds);
+  acc_launch<F>(cp.warp_acc, s, cb.acc_bases, cb.acc_entries, cb.acc_offsets, cp.K, cp.nthreads, cb.buckets, cb.head,
+                cb.tail, cb.hk, cb.tk);
   GM_CHECK_LAUNCH("k_accumulate");
   (*launches)++;
   return GM_OK;
 }
 
-// Enqueue one class's whole pipeline on `s`.
+// Enqueue one class's whole pipeline on `s`; rounds: with the affine rounds
+// (not where classes run beside each other: they share the rounds' scratch).
 template <class F>
-int batch_class_run(const BatchPlan &plan, const BatchClassPlan &cp, cudaStream_t s, const uint64_t *scalars,
-                    uint64_t *results) {
+int batch_class_run(const BatchPlan &plan, const BatchClassPlan &cp, cudaStream_t s, bool rounds,
+                    const uint64_t *scalars, uint64_t *results) {
   if (cp.count == 0) return GM_OK;
   int launches = 0;
-  int rc = batch_class_sort<F>(cp, s, scalars, &launches);
+  int rc = batch_class_sort<F>(plan, cp, s, scalars, &launches);
   if (rc) return rc;
-  rc = batch_class_accumulate<F>(plan, cp, s, &launches);
+  rounds = rounds && plan.rounds(cp);
+  if (rounds) rc = batch_class_rounds<F>(plan, cp, s, &launches);
   if (rc) return rc;
-  rc = batch_class_finish<F>(cp, s, results, &launches);
+  rc = batch_class_accumulate<F>(plan, cp, s, rounds, &launches);
+  if (rc) return rc;
+  rc = batch_class_finish<F>(plan, cp, s, rounds, results, &launches);
   count_launches(launches);
   return rc;
 }
@@ -191,8 +233,8 @@ int batch_queue_setup(BatchPlan &plan) {
   int64_t items = 0;
   for (size_t k = 0; k < plan.classes.size(); k++) {
     const BatchClassPlan &cp = plan.classes[k];
-    ClassBufs<F> cb(cp);
-    h[k] = AccClass<F>{cp.pc_table ? cp.pc_table : plan.bases, cb.entries, cb.offsets, cp.K, cp.nthreads,
+    ClassBufs<F> cb(plan, cp, plan.rounds(cp));
+    h[k] = AccClass<F>{cb.acc_bases, cb.acc_entries, cb.acc_offsets, cp.K, cp.nthreads,
                        cb.buckets, cb.head, cb.tail, cb.hk, cb.tk, items};
     if (!cp.warp_acc) items += cp.nthreads / 32;  // nthreads is a multiple of 128 then
   }
@@ -202,7 +244,8 @@ int batch_queue_setup(BatchPlan &plan) {
 }
 
 // The queued flow: every class sorts on its stream; s joins them, runs the
-// accumulation of all classes in one persistent launch, and forks the
+// affine rounds class after class and the accumulation of all classes in one
+// persistent launch, and forks the
 // classes again for their fix-ups, reductions and combinations.
 template <class F>
 int batch_run_queued(const BatchPlan &plan, cudaStream_t s, const uint64_t *scalars, uint64_t *results) {
@@ -210,12 +253,12 @@ int batch_run_queued(const BatchPlan &plan, cudaStream_t s, const uint64_t *scal
   GM_CHECK(cudaEventRecord(plan.fork, s));
   for (const auto &cp : plan.classes) {
     GM_CHECK(cudaStreamWaitEvent(cp.stream, plan.fork, 0));
-    int rc = batch_class_sort<F>(cp, cp.stream, scalars, &launches);
+    int rc = batch_class_sort<F>(plan, cp, cp.stream, scalars, &launches);
     if (rc) return rc;
     if (cp.warp_acc) {  // few entries: the class's whole pipeline beside the others
-      rc = batch_class_accumulate<F>(plan, cp, cp.stream, &launches);
+      rc = batch_class_accumulate<F>(plan, cp, cp.stream, false, &launches);
       if (rc) return rc;
-      rc = batch_class_finish<F>(cp, cp.stream, results, &launches);
+      rc = batch_class_finish<F>(plan, cp, cp.stream, false, results, &launches);
       if (rc) return rc;
     }
     GM_CHECK(cudaEventRecord(cp.sorted, cp.stream));
@@ -225,10 +268,16 @@ int batch_run_queued(const BatchPlan &plan, cudaStream_t s, const uint64_t *scal
     count_launches(launches);
     return GM_OK;
   }
+  int rc = GM_OK;
+  for (const auto &cp : plan.classes)
+    if (plan.rounds(cp)) {
+      rc = batch_class_rounds<F>(plan, cp, s, &launches);
+      if (rc) return rc;
+    }
   GM_CHECK(cudaMemsetAsync(plan.queue_ctr, 0, sizeof(uint32_t), s));
   int dev = 0, sms = 0;
   GM_CHECK(cudaGetDevice(&dev));
-  int rc = device_sm_count(dev, &sms);
+  rc = device_sm_count(dev, &sms);
   if (rc) return rc;
   const AccOccupancy occ = acc_occupancy<F>(dev, 1);
   k_accumulate_queue<F><<<(unsigned)(sms * occ.blocks), ACC_THREADS, occ.smem, s>>>(
@@ -239,7 +288,7 @@ int batch_run_queued(const BatchPlan &plan, cudaStream_t s, const uint64_t *scal
   for (const auto &cp : plan.classes) {
     if (cp.warp_acc) continue;
     GM_CHECK(cudaStreamWaitEvent(cp.stream, plan.acc_done, 0));
-    rc = batch_class_finish<F>(cp, cp.stream, results, &launches);
+    rc = batch_class_finish<F>(plan, cp, cp.stream, plan.rounds(cp), results, &launches);
     if (rc) return rc;
     GM_CHECK(cudaEventRecord(cp.done, cp.stream));
     GM_CHECK(cudaStreamWaitEvent(s, cp.done, 0));
@@ -270,7 +319,7 @@ int batch_run(const BatchPlan &plan, cudaStream_t s, const uint64_t *scalars, ui
   if (plan.classes.size() == 1 || plan.fork == nullptr) {
     // one class, or a transient plan without its own streams: in order on s
     for (const auto &cp : plan.classes) {
-      const int rc = batch_class_run<F>(plan, cp, s, scalars, results);
+      const int rc = batch_class_run<F>(plan, cp, s, true, scalars, results);
       if (rc) return rc;
     }
     return GM_OK;
@@ -279,7 +328,7 @@ int batch_run(const BatchPlan &plan, cudaStream_t s, const uint64_t *scalars, ui
   GM_CHECK(cudaEventRecord(plan.fork, s));
   for (const auto &cp : plan.classes) {
     GM_CHECK(cudaStreamWaitEvent(cp.stream, plan.fork, 0));
-    const int rc = batch_class_run<F>(plan, cp, cp.stream, scalars, results);
+    const int rc = batch_class_run<F>(plan, cp, cp.stream, false, scalars, results);
     if (rc) return rc;
     GM_CHECK(cudaEventRecord(cp.done, cp.stream));
     GM_CHECK(cudaStreamWaitEvent(s, cp.done, 0));

@@ -4,7 +4,7 @@
 namespace gm {
 template int msm_launch<Fp>(cudaStream_t, int, const uint4 *, const uint64_t *, int, const uint64_t *, int, int64_t,
                             uint64_t *, int, uint32_t *, cudaEvent_t, TailHandoff *, bool);
-template int msm_plan<Fp>(MsmLayout<Fp> &, int, int64_t, int, int, bool, int64_t);
+template int msm_plan<Fp>(MsmLayout<Fp> &, int, int64_t, int, int, bool, int64_t, bool);
 template int msm_run<Fp>(cudaStream_t, const MsmLayout<Fp> &, char *, const uint4 *, const uint64_t *, int,
                          const uint64_t *, uint64_t *, uint32_t *, cudaEvent_t, TailHandoff *, bool);
 template int batch_layouts<Fp>(BatchPlan &, int);

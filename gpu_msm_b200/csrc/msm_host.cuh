@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "msm_engine.h"
+#include "msm_affine.cuh"
 #include "msm_kernels.cuh"
 #include "msm_reduce.cuh"
 #include "msm_sort.cuh"
@@ -79,6 +80,8 @@ struct MsmLayout {
   int64_t long_cap = 0;
   bool need_pack = false;
   bool warp_acc = false;  // accumulation slices on warps
+  AffLayout al;
+  size_t o_aff = 0, o_aff_scratch = 0;
   SortLayout sl;
   RedLayout rl;
 
@@ -86,7 +89,7 @@ struct MsmLayout {
   // most_slices: bound on them, or 0;
   // level0_wave: threads of k_red_level0 resident at once
   void plan(int64_t n_, int limbs, int c, int64_t slice_threads, bool pack, int64_t level0_wave, int sms,
-            int64_t most_slices) {
+            int64_t most_slices, bool affine_rounds) {
     n = n_;
     need_pack = pack;
     dp.c = c;
@@ -111,6 +114,9 @@ struct MsmLayout {
     long_cap = nthreads / FIX_SHORT + 1;
     o_longq = cv.take<int32_t>((size_t)(1 + long_cap));
     o_err = cv.take<uint32_t>(4);
+    if (affine_rounds) al.plan<F, Carve>(&n, 1, dp.W, 1, dp.B, sms);
+    o_aff = cv.take<char>(al.bytes);
+    o_aff_scratch = cv.take<char>(al.scratch);
     o_packed = pack ? cv.take<uint4>((size_t)n * Rec<F>::U4) : 0;
     bytes = cv.off;
   }
@@ -257,7 +263,8 @@ int reduce_launch(cudaStream_t s, const RedLayout &rl, const xyzz_t<F> *buckets,
 // accumulation slice per thread of a full wave (ACC_BLOCKS_MAX blocks per SM)
 // or per warp (acc_slices); else at most that many slices.
 template <class F>
-int msm_plan(MsmLayout<F> &lay, int dev, int64_t n, int limbs, int c, bool pack, int64_t slice_threads) {
+int msm_plan(MsmLayout<F> &lay, int dev, int64_t n, int limbs, int c, bool pack, int64_t slice_threads,
+             bool affine_rounds) {
   if (limbs < 1 || limbs > MAX_SCALAR_LIMBS || n < 1 || n > (int64_t)INT32_MAX) {
     set_last_error("invalid scalar_limbs or n");
     return GM_ERR_ARG;
@@ -271,7 +278,8 @@ int msm_plan(MsmLayout<F> &lay, int dev, int64_t n, int limbs, int c, bool pack,
   if (rc) return rc;
   const int64_t most = slice_threads;
   if (slice_threads <= 0) slice_threads = (int64_t)sms * acc_blocks_per_sm<F>(dev) * ACC_THREADS;
-  lay.plan(n, limbs, c, slice_threads, pack, (int64_t)sms * level0_blocks_per_sm<F>(dev) * 128, sms, most);
+  lay.plan(n, limbs, c, slice_threads, pack, (int64_t)sms * level0_blocks_per_sm<F>(dev) * 128, sms, most,
+           affine_rounds);
   lay.rl.dev = dev;
   if ((uint64_t)n * lay.dp.W >= (1ull << 32)) {
     set_last_error("too many (point, window) entries for 32-bit offsets");
@@ -295,8 +303,9 @@ int msm_run(cudaStream_t s, const MsmLayout<F> &lay, char *ws, const uint4 *base
             TailHandoff *handoff = nullptr, bool affine = false) {
   constexpr int H = F::LIMBS / 2;  // u64 words per coordinate
   const int64_t n = lay.n;
-  auto *offsets = (uint32_t *)(ws + lay.o_offsets);
-  auto *entries = (uint32_t *)(ws + lay.o_entries);
+  auto *sorted_off = (uint32_t *)(ws + lay.o_offsets);
+  auto *sorted = (uint32_t *)(ws + lay.o_entries);
+  const uint32_t *offsets = sorted_off, *entries = sorted;
   auto *buckets = (xyzz_t<F> *)(ws + lay.o_buckets);
   auto *head = (xyzz_t<F> *)(ws + lay.o_head);
   auto *tail = (xyzz_t<F> *)(ws + lay.o_tail);
@@ -313,7 +322,7 @@ int msm_run(cudaStream_t s, const MsmLayout<F> &lay, char *ws, const uint4 *base
   {
     SortDesc sd;
     sd.n_single = n;
-    const cudaError_t e = sort_launch(s, lay.sl, ws, scalars, sd, lay.K, offsets, entries, &launches);
+    const cudaError_t e = sort_launch(s, lay.sl, ws, scalars, sd, lay.K, sorted_off, sorted, &launches);
     if (e != cudaSuccess) return record_error(e, "sort");
   }
   profile_mark(s, "sort");
@@ -325,6 +334,14 @@ int msm_run(cudaStream_t s, const MsmLayout<F> &lay, char *ws, const uint4 *base
     bases = packed;
     launches++;
     profile_mark(s, "pack");
+  }
+  if (lay.al.rounds > 0) {
+    const cudaError_t e = aff_launch<F>(s, lay.al, ws + lay.o_aff, ws + lay.o_aff_scratch, bases, entries, offsets, &launches);
+    if (e != cudaSuccess) return record_error(e, "k_affine_round");
+    profile_mark(s, "affine");
+    bases = lay.al.final_points(ws + lay.o_aff);
+    entries = nullptr;
+    offsets = lay.al.final_offsets(ws + lay.o_aff);
   }
   acc_launch<F>(lay.warp_acc, s, bases, entries, offsets, lay.K, lay.nthreads, buckets, head, tail, hk, tk);
   GM_CHECK_LAUNCH("k_accumulate");
@@ -383,11 +400,18 @@ int msm_launch(cudaStream_t s, int dev, const uint4 *bases, const uint64_t *ref_
     return GM_OK;
   }
   const int c = c_override > 0 ? c_override : default_window(sizeof(typename F::T) == sizeof(fp_t) ? 1 : 2, n, limbs);
+  // without the affine rounds where the device has no room for their scratch
   MsmLayout<F> lay;
-  int rc = msm_plan<F>(lay, dev, n, limbs, c, bases == nullptr, 0);
-  if (rc) return rc;
   char *ws = nullptr;
-  rc = pool_alloc(dev, s, lay.bytes, (void **)&ws);
+  int rc = GM_OK;
+  for (const bool rounds : {true, false}) {
+    lay = MsmLayout<F>();
+    rc = msm_plan<F>(lay, dev, n, limbs, c, bases == nullptr, 0, rounds);
+    if (rc) return rc;
+    rc = pool_alloc(dev, s, lay.bytes, (void **)&ws);
+    if (rc == GM_OK || lay.al.rounds == 0) break;
+    cudaGetLastError();  // the failed allocation
+  }
   if (rc) return rc;
   rc = msm_run<F>(s, lay, ws, bases, ref_points, to_mont, scalars, out, err_out, bases_ready,
                   handoff, affine);

@@ -356,7 +356,11 @@ GM_DEVI void cp_async16(void *smem, const void *gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem));
 }
 GM_DEVI void cp_async_commit() { asm volatile("cp.async.commit_group;"); }
-GM_DEVI void cp_async_wait_prev() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
+template <int N>
+GM_DEVI void cp_async_wait() {  // all but the N newest groups
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+GM_DEVI void cp_async_wait_prev() { cp_async_wait<1>(); }
 
 constexpr int ACC_THREADS = 128;
 template <class F>
@@ -436,8 +440,10 @@ GM_DEVI void acc_slice(const uint4 *__restrict__ bases, const uint32_t *__restri
     xyzz_t<FA> acc;
     xyzz_set_inf(acc);
     uint32_t pos = start;
-    uint32_t e_cur = __ldg(entries + pos);
-    uint32_t e_nxt = (pos + 1 < end) ? __ldg(entries + pos + 1) : 0u;
+    // no entries: the points themselves lie in bucket order
+    auto entry = [&](uint32_t i) { return entries ? __ldg(entries + i) : i << 1; };
+    uint32_t e_cur = entry(pos);
+    uint32_t e_nxt = (pos + 1 < end) ? entry(pos + 1) : 0u;
     {
       const uint4 *src = bases + (size_t)(e_cur >> 1) * Rec<F>::U4;
 #pragma unroll
@@ -453,7 +459,7 @@ GM_DEVI void acc_slice(const uint4 *__restrict__ bases, const uint32_t *__restri
         for (int q = 0; q < CH; q++) cp_async16(&stage[slot ^ 1][q][tid], src + q);
       }
       cp_async_commit();
-      const uint32_t e_after = (pos + 2 < end) ? __ldg(entries + pos + 2) : 0u;
+      const uint32_t e_after = (pos + 2 < end) ? entry(pos + 2) : 0u;
       cp_async_wait_prev();
       {
         const StagedPoint<F, CH> pt{stage[slot], tid, (e_cur & 1u) != 0};

@@ -36,7 +36,7 @@
 
 namespace gm {
 // instantiated once, in msm_g1.cu
-extern template int msm_plan<Fp>(MsmLayout<Fp> &, int, int64_t, int, int, bool, int64_t);
+extern template int msm_plan<Fp>(MsmLayout<Fp> &, int, int64_t, int, int, bool, int64_t, bool);
 extern template int msm_run<Fp>(cudaStream_t, const MsmLayout<Fp> &, char *, const uint4 *, const uint64_t *, int,
                                 const uint64_t *, uint64_t *, uint32_t *, cudaEvent_t, TailHandoff *, bool);
 }  // namespace gm
@@ -101,7 +101,7 @@ extern "C" int gm_g1_msm_device_noalloc(gm_stream_t stream, uint32_t gpu_index, 
   if (rc) return rc;
   gm::MsmLayout<Fp> lay;
   rc = gm::msm_plan<Fp>(lay, (int)gpu_index, n, scalar_limbs, NOALLOC_WINDOW_BITS, /*pack=*/true,
-                        NOALLOC_SLICE_THREADS);
+                        NOALLOC_SLICE_THREADS, /*affine_rounds=*/false);
   if (rc) return rc;
   if (lay.bytes > NOALLOC_SCRATCH_BYTES) {
     gm::set_last_error("gm_g1_msm_device_noalloc: request exceeds the fixed scratch size");

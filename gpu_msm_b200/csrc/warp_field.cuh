@@ -44,13 +44,6 @@ namespace gm {
 constexpr int32_t WM28 = (1 << 28) - 1;
 constexpr int W_FOLD = 14;  // limbs folded by the matrix product
 
-// limb k of p in 28-bit limbs
-GM_HDI constexpr int32_t p28(int k) {
-  const int j = (28 * k) / 32, s = (28 * k) % 32;
-  const uint64_t w = (uint64_t)FpConst::P(j) | ((uint64_t)FpConst::P(j + 1) << 32);
-  return (int32_t)((w >> s) & (uint64_t)WM28);
-}
-
 struct WarpTable {
   int32_t fold[W_FOLD][16];  // D_k limbs in lane order: pair l = limbs 2l+2, 2l+3; pair 7 = limbs 0, 1
   int32_t p[16];             // p
