@@ -172,23 +172,115 @@ inline void one_mont(uint64_t c[L]) {
   uint64_t one[L] = {1, 0, 0, 0, 0, 0, 0};
   to_mont(c, one);
 }
-// Montgomery-form inverse by Fermat, a^(p-2); 0 -> 0
-inline void mont_inv(uint64_t c[L], const uint64_t a[L]) {
+// a^-1 R^2 mod p, the inverse of a Montgomery-form element; 0 -> 0.  Division
+// steps of Bernstein and Yang ("Fast constant-time gcd computation and modular
+// inversion", 2019), delta from 1/2, as on the device (fp_inv_call of
+// field.cuh): 62 steps depend on the low 62 bits of f and g and multiply (f, g)
+// by a matrix over 2^62; the same matrix, with an exact division modulo p, acts
+// on (d, e), kept at d a = f R^2 and e a = g R^2.  8 limbs of 62 bits, the top
+// one signed; about 15 rounds.  One conversion of a projective G1 point took
+// 46 us with an exponentiation by p - 2 and takes 4 us.
+inline void mont_inv(uint64_t c[L], const uint64_t a_in[L]) {
+  typedef __int128 i128;
+  constexpr int N = 8;
+  constexpr uint64_t M62 = (uint64_t(1) << 62) - 1;
+  uint64_t a[L];
+  memcpy(a, a_in, sizeof(a));
+  while (geq_p(a)) sub_p(a);
   if (is_zero(a)) {
     memset(c, 0, sizeof(uint64_t) * L);
     return;
   }
-  uint64_t e[L];
-  memcpy(e, P, sizeof(e));
-  e[0] -= 2;
-  uint64_t acc[L];
-  one_mont(acc);
-  for (int i = L - 1; i >= 0; i--)
-    for (int b = 63; b >= 0; b--) {
-      mont_mul(acc, acc, acc);
-      if ((e[i] >> b) & 1) mont_mul(acc, acc, a);
+  auto cut = [](int64_t *o, const uint64_t *v) {
+    for (int k = 0; k < N; k++) {
+      const int j = 62 * k / 64, s = 62 * k % 64;
+      const u128 w = j < L ? (u128)v[j] | (u128)(j + 1 < L ? v[j + 1] : 0) << 64 : 0;
+      o[k] = (int64_t)((uint64_t)(w >> s) & M62);
     }
-  memcpy(c, acc, sizeof(acc));
+  };
+  int64_t p[N], f[N], g[N], d[N] = {0}, e[N];
+  cut(p, P);
+  cut(f, P);
+  cut(g, a);
+  cut(e, R2);
+  int64_t delta = 0;  // the steps' delta - 1/2
+  for (int it = 0; it < 22; it++) {  // 1288 steps suffice; 21 rounds hold more
+    int64_t any = 0;
+    for (int k = 0; k < N; k++) any |= g[k];
+    if (any == 0) break;
+    uint64_t f0 = (uint64_t)f[0], g0 = (uint64_t)g[0], u = 1, v = 0, q = 0, r = 1;
+    for (int s = 0; s < 62; s++) {
+      const uint64_t odd = 0 - (g0 & 1), sw = odd & ~(uint64_t)(delta >> 63);
+      // swap: (f, g) -> (g, -f), then g + f where g was odd
+      const uint64_t xf = (f0 ^ g0) & sw, xu = (u ^ q) & sw, xv = (v ^ r) & sw;
+      f0 ^= xf;
+      g0 = ((g0 ^ xf) ^ sw) - sw;
+      u ^= xu;
+      q = ((q ^ xu) ^ sw) - sw;
+      v ^= xv;
+      r = ((r ^ xv) ^ sw) - sw;
+      delta = ((delta ^ (int64_t)sw) - (int64_t)sw) + (int64_t)(1 + sw);  // -delta, or delta + 1
+      g0 = (g0 + (f0 & odd)) >> 1;
+      q += u & odd;
+      r += v & odd;
+      u <<= 1;
+      v <<= 1;
+    }
+    const int64_t su = (int64_t)u, sv = (int64_t)v, sq = (int64_t)q, sr = (int64_t)r;
+    // multiples of p that make the lowest limbs of d and e divisible, in [-2^61, 2^61)
+    const int64_t md = (int64_t)(((u * (uint64_t)d[0] + v * (uint64_t)e[0]) * PINV64) << 2) >> 2;
+    const int64_t me = (int64_t)(((q * (uint64_t)d[0] + r * (uint64_t)e[0]) * PINV64) << 2) >> 2;
+    i128 cf = 0, cg = 0, cd = 0, ce = 0;
+    for (int k = 0; k < N; k++) {
+      const int64_t fk = f[k], gk = g[k], dk = d[k], ek = e[k];
+      cf += (i128)su * fk + (i128)sv * gk;
+      cg += (i128)sq * fk + (i128)sr * gk;
+      cd += (i128)su * dk + (i128)sv * ek + (i128)md * p[k];
+      ce += (i128)sq * dk + (i128)sr * ek + (i128)me * p[k];
+      if (k > 0) {
+        f[k - 1] = (int64_t)((uint64_t)cf & M62);
+        g[k - 1] = (int64_t)((uint64_t)cg & M62);
+        d[k - 1] = (int64_t)((uint64_t)cd & M62);
+        e[k - 1] = (int64_t)((uint64_t)ce & M62);
+      }
+      cf >>= 62;
+      cg >>= 62;
+      cd >>= 62;
+      ce >>= 62;
+    }
+    f[N - 1] = (int64_t)cf;
+    g[N - 1] = (int64_t)cg;
+    d[N - 1] = (int64_t)cd;
+    e[N - 1] = (int64_t)ce;
+  }
+  // f is 1 or -1: +-d, a value within +-12 p, brought into [0, p)
+  const int64_t sg = f[0] == (int64_t)M62 ? -1 : 1;
+  int64_t t[N];
+  i128 cy = 0;
+  for (int k = 0; k < N; k++) {  // + 16 p > 0
+    cy += (i128)sg * d[k] + (i128)16 * p[k];
+    t[k] = k < N - 1 ? (int64_t)((uint64_t)cy & M62) : (int64_t)cy;
+    cy >>= 62;
+  }
+  for (int m = 16; m > 0; m >>= 1) {  // t < 32 p: subtract 16 p, 8 p, .. p where it fits
+    int64_t w[N];
+    cy = 0;
+    for (int k = 0; k < N; k++) {
+      cy += (i128)t[k] - (i128)m * p[k];
+      w[k] = k < N - 1 ? (int64_t)((uint64_t)cy & M62) : (int64_t)cy;
+      cy >>= 62;
+    }
+    if (w[N - 1] >= 0) memcpy(t, w, sizeof(t));
+  }
+  for (int k = 0; k < L; k++) {
+    const int j = 64 * k / 62, s = 64 * k % 62;
+    u128 w = (u128)(uint64_t)t[j] | (u128)(j + 1 < N ? (uint64_t)t[j + 1] : 0) << 62;
+    if (s) {
+      w >>= s;
+      if (j + 2 < N) w |= (u128)(uint64_t)t[j + 2] << (124 - s);
+    }
+    c[k] = (uint64_t)w;
+  }
 }
 
 // Fp2 (i^2 = -1)
@@ -224,10 +316,8 @@ inline void fp2_inv(Fp2 &c, const Fp2 &a) {
 }  // namespace gm_host
 
 // ---------------------------------------------------------------------------
-// Host XYZZ arithmetic for the window combination of a single MSM (the
-// serial tail: ~300 doublings).  A CPU core multiplies 446-bit numbers with
-// far lower latency than one GPU thread, so the tail runs here, stream-
-// ordered through cudaLaunchHostFunc.  Same EFD formulas as xyzz.cuh:
+// Host XYZZ arithmetic for the window combination of the blocking host-buffer
+// calls (~300 doublings on the calling thread).  Same EFD formulas as xyzz.cuh:
 // dbl-2008-s-1 and add-2008-s for a = 0, all values canonical (< p).
 // ---------------------------------------------------------------------------
 namespace gm_host {

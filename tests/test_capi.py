@@ -13,6 +13,7 @@ import pytest
 
 import gpu_msm_b200 as gm
 import oracle
+from gpu_msm_b200 import workload as wl
 from oracle import pyref
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
@@ -114,3 +115,31 @@ def test_reference_wrapper_rejects_nonpositive_n():
 def test_default_window_grows_with_n():
     ws = [gm.default_window(1, n, 5) for n in (16, 1 << 10, 1 << 16, 1 << 20)]
     assert ws == sorted(ws) and 3 <= ws[0] and ws[-1] <= 18
+
+
+def test_projective_to_affine_edge_values():
+    """The host inversion at its edges: Z = 1, 2, p - 1, values whose division steps differ in number, Z >= p
+    (an unreduced representative), Z = 0 (infinity); and Fp2 norms."""
+    p, r = wl.P_MODULUS, (1 << 448) % wl.P_MODULUS
+    rng = np.random.default_rng(11)
+    zs = [1, 2, 3, r, p - 1, p - 2, p // 2, 1 << 445, (1 << 62) + 1, p + 1, p + (1 << 100), 4 * p + 5]
+    zs += [int.from_bytes(rng.bytes(55), "little") for _ in range(40)]
+    proj = np.zeros(len(zs), dtype=gm.G1P)
+    for i, z in enumerate(zs):
+        proj["X"][i], proj["Y"][i], proj["Z"][i] = (wl.int_to_limbs(v, 7) for v in (7 * r % p, 11 * r % p, z))
+    got = gm.projective_to_affine(proj, 1)
+    for i, z in enumerate(zs):
+        zi = pow(z, -1, p) * r * r % p  # inverse of the Montgomery form
+        for name, v in (("x", 7), ("y", 11)):
+            want = v * r * zi * pow(r, -1, p) % p
+            assert np.array_equal(got[name][i], wl.int_to_limbs(want, 7)), (i, name)
+    proj2 = np.zeros(3, dtype=gm.G2P)
+    for i, (a, b) in enumerate([(5, 0), (0, 9), (p - 3, 1 << 300)]):
+        proj2["X"][i, 0] = wl.int_to_limbs(r, 7)
+        proj2["Z"][i, 0], proj2["Z"][i, 1] = wl.int_to_limbs(a * r % p, 7), wl.int_to_limbs(b * r % p, 7)
+    got2 = gm.projective_to_affine(proj2, 2)
+    for i, (a, b) in enumerate([(5, 0), (0, 9), (p - 3, 1 << 300)]):
+        n = pow(a * a + b * b, -1, p)
+        assert np.array_equal(got2["x"][i, 0], wl.int_to_limbs(a * n * r % p, 7))
+        assert np.array_equal(got2["x"][i, 1], wl.int_to_limbs(-b * n * r % p, 7))
+    assert bool(gm.projective_to_affine(np.zeros(1, dtype=gm.G1P), 1)["infinity"][0])
