@@ -27,9 +27,9 @@ namespace gm {
 
 constexpr int W_THREADS = 128;    // block of the kernels with one warp per work item
 constexpr int SUM_WARPS = 8;      // warps of a block sum
-constexpr int COMBINE_WARPS = 8;  // groups of windows of a window combination
+constexpr int COMBINE_WARPS = 8;  // groups of windows of a window combination, a warp each, beside the chain's warps
 template <class F>
-constexpr int COMBINE_THREADS = 32 * (COMBINE_WARPS > Chain<F>::WARPS ? COMBINE_WARPS : Chain<F>::WARPS);
+constexpr int COMBINE_THREADS = 32 * (COMBINE_WARPS + Chain<F>::WARPS);
 constexpr int W_FILL = 16;        // warps per SM that keep its schedulers busy with dependent point operations
 constexpr int ACC_WARP_MIN = 4;    // entries of a slice on a warp, at least
 constexpr int ACC_WARP_MAX = 16;   // and at most; above W_SLICES slices of these, threads take the slices
@@ -52,7 +52,7 @@ __global__ void __launch_bounds__(W_THREADS) k_accumulate_warp(
   using W = WF<F>;
   using E = typename W::E;
   w_setup();
-  const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t t = (int64_t)blockIdx.x * (W_THREADS / 32) + w_warp();
   if (t >= nslices) return;
   const uint32_t M = __ldg(offsets + K);
   const uint64_t chunk64 = ((uint64_t)M + nslices - 1) / nslices;
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(W_THREADS) k_red_level0_warp(const xyzz_t<F> *
                                                                int L0, int nseg0, xyzz_t<F> *__restrict__ X, int M,
                                                                xyzz_t<F> *__restrict__ A0) {
   w_setup();
-  const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t t = (int64_t)blockIdx.x * (W_THREADS / 32) + w_warp();
   if (t >= G * nseg0) return;
   const int64_t g = t / nseg0;
   const int s = (int)(t % nseg0);
@@ -176,7 +176,7 @@ template <class F>
 __global__ void __launch_bounds__(W_THREADS) k_red_level1(const xyzz_t<F> *__restrict__ A0, int64_t G, int nseg0,
                                                           int L1, int nseg1, int L0, xyzz_t<F> *__restrict__ X, int M) {
   w_setup();
-  const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t t = (int64_t)blockIdx.x * (W_THREADS / 32) + w_warp();
   if (t >= G * nseg1) return;
   const int64_t g = t / nseg1;
   const int s = (int)(t % nseg1);
@@ -201,7 +201,7 @@ __global__ void __launch_bounds__(32 * SUM_WARPS) k_red_sum(const xyzz_t<F> *__r
   const int i = (int)(blockIdx.x % nout);
   const int j1 = min(N, (i + 1) * chunk);
   wpt<F> acc = w_inf<F>();
-  for (int j = i * chunk + (threadIdx.x >> 5); j < j1; j += SUM_WARPS) acc = w_addp<F>(acc, w_load_pt<F>(in + g * N + j));
+  for (int j = i * chunk + w_warp(); j < j1; j += SUM_WARPS) acc = w_addp<F>(acc, w_load_pt<F>(in + g * N + j));
   acc = w_block_sum<F>(acc, SUM_WARPS, w_smem + w_smem_bytes<F>(SUM_WARPS) / 4);
   if (threadIdx.x < 32) w_store_pt<F>(out + blockIdx.x, acc);
 }
@@ -228,7 +228,7 @@ __global__ void __launch_bounds__(W_THREADS) k_fixup_split(const uint32_t *__res
                                                            uint32_t *__restrict__ err, int32_t *__restrict__ long_q,
                                                            int64_t long_cap) {
   w_setup();
-  const int64_t t = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int64_t t = (int64_t)blockIdx.x * (W_THREADS / 32) + w_warp();
   if (t >= nslices) return;
   const int32_t k = __ldg(tail_key + t);
   if (k < 0) return;
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(32 * SUM_WARPS) k_fixup_long(const uint32_t *_
   const int64_t n_long = min((int64_t)long_q[0], long_cap);
   if ((int64_t)blockIdx.x >= n_long) return;
   w_setup();
-  const int w = threadIdx.x >> 5;
+  const int w = w_warp();
   const uint32_t M = __ldg(offsets + K);
   const uint64_t chunk64 = ((uint64_t)M + nslices - 1) / nslices;
   const uint64_t chunk = chunk64 > 0 ? chunk64 : 1u;
@@ -300,11 +300,15 @@ __global__ void __launch_bounds__(32 * SUM_WARPS) k_fixup_long(const uint32_t *_
 // Window combination on the device, one block per MSM: result = sum_w
 // 2^(c w) S_w by Horner; homogeneous projective output (u64 limbs,
 // Montgomery).  The c (W - 1) doublings of the top window are one serial
-// chain, run by the block's warps together (xyzz_chain.cuh); the additions
-// are kept off it: every warp combines W / COMBINE_WARPS windows, all at once,
-// and the chain takes in the warps' sums.  out_index (optional) maps MSM i to
-// its result slot.  affine: an affine point of the reference's layout instead
-// (infinity flag in the word after the coordinates).
+// chain, run by Chain<F>::WARPS warps together (xyzz_chain.cuh).  The additions
+// are kept off it: each of COMBINE_WARPS other warps combines a group of q
+// windows, while the chain already works on the top 1 to q windows, and the
+// chain takes in one sum every c q doublings (B200, against groups first and
+// the chain after them: G1 1024 points 0.42 -> 0.39 ms, G2 1500 points
+// 0.82 -> 0.65 ms, the chain's Fp2 products on 8 warps included).
+// out_index (optional) maps MSM i to its result slot.  affine: an affine point
+// of the reference's layout instead (infinity flag in the word after the
+// coordinates).
 // ---------------------------------------------------------------------------
 template <class F>
 __global__ void __launch_bounds__(COMBINE_THREADS<F>) k_combine(const xyzz_t<F> *__restrict__ S, int W, int c,
@@ -314,37 +318,50 @@ __global__ void __launch_bounds__(COMBINE_THREADS<F>) k_combine(const xyzz_t<F> 
   constexpr int PT = w_pt_words<F>(), LW = WP::LW;
   w_setup();
   const int64_t i = blockIdx.x;
-  const int w = threadIdx.x >> 5;
-  const int q = (W + COMBINE_WARPS - 1) / COMBINE_WARPS;
-  int32_t *sums = w_smem + w_smem_bytes<F>(COMBINE_WARPS) / 4;
-  int32_t *io = sums + COMBINE_WARPS * PT, *ctl = io + 3 * LW;
-  // the chain works in the scratch of warps 1 and up, which are done by then
-  int32_t *work = w_smem + W_TABLE_WORDS + w_scratch_words<F>();
-  static_assert(chain_words<F>() <= (COMBINE_WARPS - 1) * w_scratch_words<F>(), "chain scratch");
-  wpt<F> res = w_inf<F>();
-  if (w < COMBINE_WARPS) {
-    for (int j = min(W, (w + 1) * q) - 1; j >= w * q; j--) {
-      if (!res.inf)
-        for (int k = 0; k < c; k++) res = w_dbl<F>(res);
-      res = w_addp<F>(res, w_load_pt<F>(S + i * W + j));
-    }
-    w_put_pt<F>(sums + w * PT, res);
+  const int w = w_warp();
+  constexpr int NCH = Chain<F>::WARPS, LEAD = COMBINE_WARPS;  // the chain's warps are LEAD .. LEAD + NCH - 1
+  // top: the highest window with anything in it (scalars rarely reach the last ones)
+  int top = 0;
+  for (int b = 0; b < W; b += 32) {
+    const int j = b + (int)(threadIdx.x & 31u);
+    const unsigned m = __ballot_sync(0xffffffffu, j < W && !F::is_zero_raw(S[i * W + j].ZZ));
+    if (m) top = b + 31 - __clz(m);
   }
-  __syncthreads();
-  if (w >= Chain<F>::WARPS) return;
-  int top = (W + q - 1) / q - 1;
-  while (top > 0 && sums[top * PT + 4 * LW] != 0) top--;  // windows at infinity
-  res = w_get_pt<F>(sums + top * PT);
-  for (int j = top - 1; j >= 0; j--) {
-    if (w == 0) {
-      if (threadIdx.x == 0) ctl[0] = res.inf ? 1 : 0;
+  const int q = max(1, (top + COMBINE_WARPS - 1) / COMBINE_WARPS);
+  const int groups = top / q;  // the windows from groups * q to top are the chain's own
+  int32_t *sums = w_smem + w_smem_bytes<F>(LEAD + 1) / 4;
+  int32_t *io = sums + COMBINE_WARPS * PT, *ctl = io + 3 * LW, *work = ctl + 4;
+  wpt<F> res = w_inf<F>();
+  if (w <= LEAD) {
+    const int lo = w < LEAD ? w * q : groups * q, hi = w < LEAD ? (w + 1) * q : top + 1;
+    if (w == LEAD || w < groups)
+      for (int j = hi - 1; j >= lo; j--) {
+        if (!res.inf)
+          for (int k = 0; k < c; k++) res = w_dbl<F>(res);
+        res = w_addp<F>(res, w_load_pt<F>(S + i * W + j));
+      }
+  }
+  if (w < LEAD) {
+    w_put_pt<F>(sums + w * PT, res);
+    asm volatile("bar.arrive 2, %0;" ::"n"(COMBINE_THREADS<F>) : "memory");
+    return;
+  }
+  bool waited = false;
+  auto group_sums = [&] {  // once: the groups' warps are done
+    if (!waited) asm volatile("bar.sync 2, %0;" ::"n"(COMBINE_THREADS<F>) : "memory");
+    waited = true;
+  };
+  for (int j = groups - 1; j >= 0; j--) {
+    if (w == LEAD) {
+      if (threadIdx.x == 32 * LEAD) ctl[0] = res.inf ? 1 : 0;
       WP::put(io, res.X);
       WP::put(io + LW, res.Y);
       WP::put(io + 2 * LW, WP::one());
     }
-    asm volatile("bar.sync 1, %0;" ::"n"(32 * Chain<F>::WARPS) : "memory");
-    if (ctl[0] == 0) chain_dbl<F>(c * q, io, work);
-    if (w == 0) {
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * NCH) : "memory");
+    if (ctl[0] == 0) chain_dbl<F>(c * q, LEAD, io, work);
+    group_sums();
+    if (w == LEAD) {
       if (!res.inf) {
         const typename WP::E L = WP::get(io + 2 * LW);
         res.X = WP::get(io);
@@ -359,9 +376,10 @@ __global__ void __launch_bounds__(COMBINE_THREADS<F>) k_combine(const xyzz_t<F> 
       }
       res = w_addp<F>(res, w_get_pt<F>(sums + j * PT));
     }
-    asm volatile("bar.sync 1, %0;" ::"n"(32 * Chain<F>::WARPS) : "memory");
+    asm volatile("bar.sync 1, %0;" ::"n"(32 * NCH) : "memory");
   }
-  if (w > 0) return;
+  group_sums();  // where there are no groups the barrier is still to be completed
+  if (w > LEAD) return;
   constexpr int H = F::LIMBS / 2;
   const int g = w_group();
   const int64_t slot = out_index ? (int64_t)__ldg(out_index + i) : i;
@@ -373,7 +391,7 @@ __global__ void __launch_bounds__(COMBINE_THREADS<F>) k_combine(const xyzz_t<F> 
     typename F::T v = WP::canon(WP::mul(WP::pick(g, res.X, res.Y, res.X, res.Y), t));
     uint64_t *o = out + slot * (2 * H + 1);
     if (g < 2 && w_lane() == 0) store_ref<F>(o + g * H, v);
-    if (threadIdx.x == 0) o[2 * H] = res.inf ? 1u : 0u;
+    if (threadIdx.x == 32 * LEAD) o[2 * H] = res.inf ? 1u : 0u;
     return;
   }
   // (X ZZZ, Y ZZ, ZZ ZZZ); infinity is (0, 0, 0)
@@ -387,7 +405,7 @@ __global__ void __launch_bounds__(COMBINE_THREADS<F>) k_combine(const xyzz_t<F> 
 
 template <class F>
 constexpr int combine_smem() {
-  return w_sum_smem<F>(COMBINE_WARPS) + 4 * (3 * WF<F>::LW + 4);
+  return w_smem_bytes<F>(COMBINE_WARPS + 1) + 4 * (COMBINE_WARPS * w_pt_words<F>() + 3 * WF<F>::LW + 4 + chain_words<F>());
 }
 
 // ---------------------------------------------------------------------------

@@ -117,6 +117,9 @@ constexpr int w_smem_bytes(int warps) {
 
 extern __shared__ __align__(16) int32_t w_smem[];
 
+// Index of the warp in its block, through a shuffle: the compiler then knows
+// branches on it as uniform and leaves out their reconvergence.
+GM_DEVI int w_warp() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
 GM_DEVI int w_lane() { return (int)(threadIdx.x & 7u); }
 GM_DEVI int w_group() { return (int)((threadIdx.x >> 3) & 3u); }
 GM_DEVI const WarpTable &w_table() { return *reinterpret_cast<const WarpTable *>(w_smem); }

@@ -173,7 +173,7 @@ constexpr int w_sum_smem(int warps) {
 // s: warps * w_pt_words<F>() words.  Every warp of the block calls it.
 template <class F>
 GM_DEVI wpt<F> w_block_sum(wpt<F> v, int warps, int32_t *s) {
-  const int w = threadIdx.x >> 5;
+  const int w = w_warp();
   for (int h = warps >> 1; h >= 1; h >>= 1) {
     if (w >= h && w < 2 * h) w_put_pt<F>(s + (w - h) * w_pt_words<F>(), v);
     __syncthreads();
