@@ -161,6 +161,7 @@ template <bool FIRST>
 struct AffWalk {
   const uint32_t *entries, *off_in, *off_out;
   uint32_t in0;
+  int64_t k0, k1;  // the chunk's buckets
   int64_t k;
   uint32_t ob, oe, ib, ie;
   GM_DEVI void start(int64_t k_) {
@@ -184,7 +185,11 @@ struct AffWalk {
     return r;
   }
   GM_DEVI AffPair forward(uint32_t j) {
-    while (j >= oe) {
+    for (int s = 0; j >= oe; s++) {
+      if (s == 4) {  // a run of empty buckets
+        start(k + bucket_of(off_out + k, k1 - k, j));
+        break;
+      }
       k++;
       ob = oe;
       oe = __ldg(off_out + k + 1);
@@ -194,7 +199,11 @@ struct AffWalk {
     return at(j);
   }
   GM_DEVI AffPair backward(uint32_t j) {
-    while (j < ob) {
+    for (int s = 0; j < ob; s++) {
+      if (s == 4) {
+        start(k0 + bucket_of(off_out + k0, k - k0, j));
+        break;
+      }
       k--;
       oe = ob;
       ob = __ldg(off_out + k);
@@ -267,7 +276,7 @@ __global__ void __launch_bounds__(AFF_THREADS, AFF_BLOCKS<F>)
   const uint64_t start64 = (uint64_t)o0 + (uint64_t)t * chunk;
   if (start64 >= o1) return;
   const uint32_t end = (uint32_t)min(start64 + chunk, (uint64_t)o1);
-  AffWalk<FIRST> walk{entries, off_in, off_out, FIRST ? 0u : __ldg(off_in + k0)};
+  AffWalk<FIRST> walk{entries, off_in, off_out, FIRST ? 0u : __ldg(off_in + k0), k0, k1};
   walk.start(k0 + bucket_of(off_out + k0, k1 - k0, (uint32_t)start64));
   out -= (size_t)(local_out ? o0 : 0u) * U4;
 

@@ -350,6 +350,16 @@ GM_DEVI int64_t bucket_of(const uint32_t *__restrict__ offsets, int64_t K, uint3
   return lo;
 }
 
+// The bucket of position pos, from bucket k < K at or before it: the next ones
+// first, then a search.  The windows above a scalar's top bits are whole runs
+// of empty buckets, 2^(c-1) each, in the middle of a batch's keys.
+GM_DEVI int64_t seek_bucket(const uint32_t *__restrict__ offsets, int64_t k, int64_t K, uint32_t pos) {
+#pragma unroll 1
+  for (int s = 0; s < 4; s++, k++)
+    if (__ldg(offsets + k + 1) > pos) return k;
+  return k + bucket_of(offsets + k, K - k, pos);
+}
+
 // Asynchronous 16-byte global -> shared copy (cp.async, L2 only).
 GM_DEVI void cp_async16(void *smem, const void *gmem) {
   const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
@@ -480,8 +490,7 @@ GM_DEVI void acc_slice(const uint4 *__restrict__ bases, const uint32_t *__restri
           tk = (int32_t)k;
         }
         if (pos == end) break;
-        k++;
-        while (__ldg(offsets + k + 1) <= pos) k++;
+        k = seek_bucket(offsets, k + 1, K, pos);
         bend = __ldg(offsets + k + 1);
         owns = true;
         xyzz_set_inf(acc);

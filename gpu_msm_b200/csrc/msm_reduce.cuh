@@ -93,8 +93,7 @@ __global__ void __launch_bounds__(W_THREADS) k_accumulate_warp(
           tk = (int32_t)k;
         }
         if (pos == end) break;
-        k++;
-        while (__ldg(offsets + k + 1) <= pos) k++;
+        k = seek_bucket(offsets, k + 1, K, pos);
         bend = __ldg(offsets + k + 1);
         owns = true;
         acc = w_inf<F>();
