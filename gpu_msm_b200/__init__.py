@@ -632,10 +632,13 @@ class ResidentBases:
 
     def windows_for(self, sizes, scalar_limbs: int = 5):
         """Per-MSM window widths to pass to a plan: 0 (the library picks the
-        cheapest fixed-base table) when the set has tables, else the tuned
-        widths."""
+        cheapest fixed-base table) when the set has tables; one width for all
+        of a small batch; else the tuned widths."""
         if self.precomputed:
             return [0] * len(sizes)
+        sizes = np.asarray(sizes, dtype=np.int64)
+        if len(sizes) > 1 and int(sizes.sum()) <= BATCH_ONE_CLASS:
+            return [batch_window(sizes, scalar_limbs)] * len(sizes)
         return [tuned_window(self.group, int(s), scalar_limbs) for s in sizes]
 
     def msm(self, scalars, offset: int = 0, n: int = None, window_bits: int = 0, out=None, stream=None):
@@ -695,6 +698,26 @@ def tuned_params(group: int, n: int, scalar_limbs: int = 5):
     if v is not None:
         return int(v), 1, 4
     return default_window(group, n, scalar_limbs), 1, 4
+
+
+# Up to this many points in all, a batch takes one window width.  Every width
+# is a class with its own sort, fix-up and reduction, which a small batch does
+# not fill the GPU with.  B200, tuned widths per MSM -> one width: 20 G2 MSMs of
+# 2^6..2^12 points (25 k in all) 4.84 -> 3.60 ms, 20 such G1 MSMs 2.14 -> 1.50 ms,
+# 40 G1 MSMs of 2^10..2^14 (209 k) 5.43 -> 4.85 ms; 256 G2 MSMs of 2^8..2^12
+# (357 k) 26.6 -> 29.4 ms, so not there.
+BATCH_ONE_CLASS = 1 << 18
+
+
+def batch_window(sizes, scalar_limbs: int = 5) -> int:
+    """One window width for a small batch: 10 products per (point, window) and
+    38 per bucket, least over all its MSMs together."""
+    bits = min(64 * scalar_limbs, 299)
+    total, count = int(np.sum(sizes)), len(sizes)
+
+    def cost(c):
+        return 10 * total * (bits // c + 1) + 38 * count * (64 * scalar_limbs // c + 1) * 2 ** (c - 1)
+    return min(range(3, 13), key=cost)
 
 
 def tuned_window(group: int, n: int, scalar_limbs: int = 5) -> int:

@@ -101,7 +101,7 @@ def main():
     args = ap.parse_args()
     dev = torch.device("cuda", 0)
     reps = 2 if args.quick else 3
-    ppc = 1 << (17 if args.quick else 18)
+    ppc = 1 << (18 if args.quick else 20)
     t0 = time.time()
     g1, d1 = tune_group(1, 4, 20, ppc, reps, dev)
     g2, d2 = tune_group(2, 4, 18, ppc, reps, dev)

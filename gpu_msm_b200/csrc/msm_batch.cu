@@ -97,6 +97,49 @@ void plan_rounds(gm::BatchPlan &plan) {
   }
 }
 
+// Window widths of MSMs over fixed-base tables (0 without a table for the
+// scalars).  An MSM costs 10 products per (point, window) and, with its single
+// bucket set, 50 per bucket (two additions of 14 and the upper levels' share).
+// A further class of a batch costs about TABLE_CLASS products' time whatever
+// its size (its own sort, fix-up and reduction launches, 0.2 ms), so all take
+// the table that is best for the whole batch unless the best one for each
+// saves more.  B200, each MSM's own best at 28 per bucket -> this rule: 40 MSMs
+// of 2^8..2^14 points over widths 11 and 14 3.10 -> 2.52 ms, 24 of 2^10..2^16
+// 5.67 -> 5.38 ms.
+constexpr double TABLE_CLASS = 4e6;
+std::vector<int> choose_tables(const gm_bases *b, int scalar_limbs, int count, const int64_t *sizes) {
+  std::vector<int> each(count, 0);
+  double best_all = 0, each_sum = 0;
+  int c_all = 0;
+  std::map<int, int> used;
+  for (int i = 0; i < count; i++) {
+    double best = 0;
+    for (const auto &t : b->tables) {
+      if (t.W < gm::windows_for(t.c, scalar_limbs)) continue;
+      const double cost = 10.0 * (double)sizes[i] * (64.0 * scalar_limbs / t.c) + 50.0 * (double)(1 << (t.c - 1));
+      if (each[i] == 0 || cost < best) {
+        best = cost;
+        each[i] = t.c;
+      }
+    }
+    each_sum += best;
+    if (each[i]) used[each[i]]++;
+  }
+  if (used.size() < 2) return each;
+  for (const auto &t : b->tables) {
+    if (t.W < gm::windows_for(t.c, scalar_limbs)) continue;
+    double cost = 0;
+    for (int i = 0; i < count; i++)
+      cost += 10.0 * (double)sizes[i] * (64.0 * scalar_limbs / t.c) + 50.0 * (double)(1 << (t.c - 1));
+    if (c_all == 0 || cost < best_all) {
+      best_all = cost;
+      c_all = t.c;
+    }
+  }
+  if (best_all <= each_sum + TABLE_CLASS * (double)(used.size() - 1)) each.assign(count, c_all);
+  return each;
+}
+
 // Validates the batch, groups MSMs by window width and computes each class's
 // layout; d64[k] / idx[k] receive class k's descriptors
 // (point_start | base_off | sc_off, and out_index | tile_first).
@@ -110,6 +153,7 @@ int build_classes(const gm_bases *b, int scalar_limbs, int count, const int64_t 
   if (!b || count <= 0 || !sizes || scalar_limbs < 1 || scalar_limbs > gm::MAX_SCALAR_LIMBS) return gm::GM_ERR_ARG;
   int rc = gm::select_device((uint32_t)b->dev);
   if (rc) return rc;
+  const std::vector<int> table_c = choose_tables(b, scalar_limbs, count, sizes);
   std::map<int, std::vector<int>> by_c;
   std::vector<int64_t> sc_row(count + 1, 0);
   for (int i = 0; i < count; i++) {
@@ -120,20 +164,7 @@ int build_classes(const gm_bases *b, int scalar_limbs, int count, const int64_t 
     }
     sc_row[i + 1] = sc_row[i] + sizes[i];
     int c = window_bits && window_bits[i] > 0 ? window_bits[i] : 0;
-    if (c == 0 && !b->tables.empty()) {
-      // with fixed-base tables an MSM costs ~10 products per (point, non-zero
-      // window) plus 2 additions (28 products) per bucket of its single
-      // bucket set; take the cheapest table
-      double best = 0;
-      for (const auto &t : b->tables) {
-        if (t.W < gm::windows_for(t.c, scalar_limbs)) continue;
-        const double cost = 10.0 * (double)sizes[i] * (64.0 * scalar_limbs / t.c) + 28.0 * (double)(1 << (t.c - 1));
-        if (c == 0 || cost < best) {
-          best = cost;
-          c = t.c;
-        }
-      }
-    }
+    if (c == 0) c = table_c[i];
     if (c == 0) c = gm::default_window(b->group, sizes[i], scalar_limbs);
     if (c < 2 || c > 20) {
       gm::set_last_error("window width out of range");

@@ -257,24 +257,30 @@ int pool_alloc(int dev, cudaStream_t s, size_t bytes, void **ptr) {
 
 // ---------------------------------------------------------------------------
 // window selection (cost model in multiplication units)
-//   accumulation: 10 mults per (point, non-zero window)     (madd 8M+2S)
-//   reduction:    ~2.7 full adds of 14 mults per bucket      (running sums)
-//   combine:      c doublings (9 mults) per window, on one thread: weighted
+//   accumulation: 10 per (point, non-zero window) (madd 8M+2S), 7 where rounds
+//                 of affine additions run first (about 3 M entries up)
+//   reduction:    two full additions of 14 mults per bucket and the upper
+//                 levels: 38; 48 (G1) and 60 (G2) against the cheaper entries
+//   combine:      c doublings (9 mults) per window in one chain: weighted
 //                 by the serial latency against a wave of the whole GPU.
+// B200, best width measured (the model's where it differs): G1 2^18 12, 400000
+// 12, 600000 15, 2^20 15, 2^21 15; G2 130000 12, 2^18 12, 2^19 14; with 10 and 38
+// throughout the model took 15 for G1 2^18 (4.12 against 3.87 ms), 16 for 2^20
+// (11.3 / 10.9), 15 for G2 2^18 (10.5 / 9.5).
 // ---------------------------------------------------------------------------
 static int windows_for(int c, int limbs) { return (64 * limbs) / c + 1; }
 
 int default_window(int group, int64_t n, int limbs) {
-  (void)group;
   if (n <= 0) return 4;
-  const int bits = std::min(64 * limbs, 300);
+  const int sbits = std::min(64 * limbs, 299);  // scalars below r have 299 significant bits
+  const bool rounds = (double)n * sbits >= 3e6 * 12;
   double best = 1e300;
   int best_c = 4;
   for (int c = 3; c <= 18; c++) {
     const int W = windows_for(c, limbs);
-    const int Weff = (bits + c) / c;
-    const double acc = 10.0 * (double)n * Weff;
-    const double red = 38.0 * (double)W * std::ldexp(1.0, c - 1);
+    const int Weff = sbits / c + 1;
+    const double acc = (rounds ? 7.0 : 10.0) * (double)n * Weff;
+    const double red = (rounds ? (group == 1 ? 48.0 : 60.0) : 38.0) * (double)W * std::ldexp(1.0, c - 1);
     const double tail = 9.0 * c * Weff * 2000.0;
     // Hot buckets: a top window of few bits puts all n of its entries into a
     // handful of buckets, and a full top window (c bits, so digits above
@@ -282,8 +288,6 @@ int default_window(int group, int64_t n, int limbs) {
     // n/2 entries; both mean long fix-up runs and contended sort counters
     // (G1 2^17: c = 11, 2 top bits, 0.32 ms more fix-up and sort than c = 12;
     // G2 2^16: c = 11 0.63 ms, c = 13 (full top window) 0.31 ms more).
-    // Scalars below r have 299 significant bits.
-    const int sbits = std::min(64 * limbs, 299);
     const int top_bits = sbits - c * ((sbits + c - 1) / c - 1);
     const double hot = (top_bits <= 3 || top_bits >= c) ? 40.0 * (double)n : top_bits <= 6 ? 20.0 * (double)n : 0.0;
     const double cost = acc + red + tail + hot;

@@ -117,3 +117,54 @@ def test_batch_class(cuda, group, count, lo, hi, tabled):
             assert oracle.same_point(res[i:i + 1], oracle.generator_multiple(w, group=group)), i
     plan.close()
     table.close()
+
+
+def test_batch_over_runs_of_empty_buckets(cuda):
+    """Scalars of 100 bits in 5 limbs: most windows of every MSM are empty, in the middle of the batch's keys."""
+    n, count, group, c = 1 << 15, 9, 1, 12
+    logs = wl.make_base_logs(n, seed=15)
+    table = gm.ResidentBases(gm.generator_mul_batch(dev(logs, cuda), group=group), group=group)
+    sizes = np.array([n - 7 * i for i in range(count)], dtype=np.int64)
+    sc = wl.make_scalars(int(sizes.sum()), seed=16)
+    sc[:, 2:] = 0
+    sc[:, 1] &= np.uint64((1 << 36) - 1)
+    sc[:: 1000, 4] = 1  # and a few full-width ones
+    want = wl.expected_logs(sizes, sc, logs)
+    out = gm.BatchPlan(table, sizes, window_bits=np.full(count, c, dtype=np.int32)).run(dev(sc, cuda))
+    torch.cuda.synchronize()
+    res = oracle.proj_to_affine(gm.to_numpy_proj(out, group), group)
+    for i, w in enumerate(want):
+        assert oracle.same_point(res[i:i + 1], oracle.generator_multiple(w, group=group)), i
+
+
+@pytest.mark.parametrize("sizes,one", [([5, 300, 17, 4000], True), ([1 << 17, 1 << 17, 7], False)])
+def test_small_batches_take_one_width(cuda, sizes, one):
+    """A small batch is one class, exact; a large one keeps the tuned widths."""
+    n = max(sizes)
+    logs = wl.make_base_logs(n, seed=21)
+    table = gm.ResidentBases(gm.generator_mul_batch(dev(logs, cuda), group=1), group=1)
+    plan = gm.BatchPlan(table, sizes)
+    assert (len(plan.classes()) == 1) == one
+    sc = wl.make_scalars(sum(sizes), seed=22)
+    out = plan.run(dev(sc, cuda))
+    torch.cuda.synchronize()
+    res = oracle.proj_to_affine(gm.to_numpy_proj(out, 1), 1)
+    for i, w in enumerate(wl.expected_logs(sizes, sc, logs)):
+        assert oracle.same_point(res[i:i + 1], oracle.generator_multiple(w)), i
+
+
+def test_tables_of_small_and_mixed_batches(cuda):
+    """Over two tables: the whole batch on one of them, or each MSM on its own best."""
+    n = 1 << 16
+    logs = wl.make_base_logs(n, seed=31)
+    table = gm.ResidentBases(gm.generator_mul_batch(dev(logs, cuda), group=1), group=1).precompute(6).precompute(14)
+    for sizes, classes in (([20, 30, 25], 1), ([60000, 50000], 1), ([60000] + [20] * 40, 2)):
+        plan = gm.BatchPlan(table, sizes)
+        assert len(plan.classes()) == classes, plan.classes()
+        sc = wl.make_scalars(sum(sizes), seed=32)
+        out = plan.run(dev(sc, cuda))
+        torch.cuda.synchronize()
+        res = oracle.proj_to_affine(gm.to_numpy_proj(out, 1), 1)
+        for i, w in enumerate(wl.expected_logs(sizes, sc, logs)):
+            assert oracle.same_point(res[i:i + 1], oracle.generator_multiple(w)), i
+        plan.close()
