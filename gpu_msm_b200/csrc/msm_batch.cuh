@@ -179,8 +179,8 @@ int batch_class_finish(const BatchPlan &plan, const BatchClassPlan &cp, cudaStre
   rc = reduce_launch<F>(s, cp.rl, cb.buckets, cb.acc_offsets, cp.ws, &src, launches);
   if (rc) return rc;
   // precomputed mode: one window per MSM, so the combination is a conversion
-  k_combine<F><<<(unsigned)cp.count, COMBINE_THREADS<F>, combine_smem<F>(), s>>>(
-      src, cp.pc_stride ? 1 : cp.dp.W, cp.c, cb.out_index, results, false);
+  launch_after(
+      k_combine<F>, (unsigned)cp.count, COMBINE_THREADS<F>, combine_smem<F>(), s, src, cp.pc_stride ? 1 : cp.dp.W, cp.c, cb.out_index, results, false);
   GM_CHECK_LAUNCH("k_combine");
   (*launches)++;
   return GM_OK;

@@ -174,8 +174,8 @@ static void acc_launch(bool warp, cudaStream_t s, const uint4 *bases, const uint
                        xyzz_t<F> *tail, int32_t *hk, int32_t *tk) {
   if (warp) {
     constexpr int WPB = W_THREADS / 32;
-    k_accumulate_warp<F><<<(unsigned)((nthreads + WPB - 1) / WPB), W_THREADS, w_smem_bytes<F>(WPB), s>>>(
-        bases, entries, offsets, K, nthreads, buckets, head, tail, hk, tk);
+    launch_after(k_accumulate_warp<F>, (unsigned)((nthreads + WPB - 1) / WPB), W_THREADS, w_smem_bytes<F>(WPB), s,
+                 bases, entries, offsets, K, nthreads, buckets, head, tail, hk, tk);
     return;
   }
   const unsigned grid = (unsigned)((nthreads + ACC_THREADS - 1) / ACC_THREADS);
@@ -208,10 +208,10 @@ template <class F>
 int fixup_launch(cudaStream_t s, const uint32_t *offsets, int64_t K, int64_t nthreads, xyzz_t<F> *buckets,
                  const xyzz_t<F> *head, const xyzz_t<F> *tail, const int32_t *hk, const int32_t *tk, uint32_t *err,
                  int32_t *long_q, int64_t long_cap, int *launches) {
-  k_fixup_split<F><<<grid_for(nthreads, W_THREADS / 32), W_THREADS, w_smem_bytes<F>(W_THREADS / 32), s>>>(
-      offsets, K, nthreads, buckets, head, tail, hk, tk, err, long_q, long_cap);
+  launch_after(k_fixup_split<F>, grid_for(nthreads, W_THREADS / 32), W_THREADS, w_smem_bytes<F>(W_THREADS / 32), s,
+               offsets, K, nthreads, buckets, head, tail, hk, tk, err, long_q, long_cap);
   GM_CHECK_LAUNCH("k_fixup_split");
-  k_fixup_long<F><<<FIX_LONG_BLOCKS, 32 * SUM_WARPS, w_sum_smem<F>(SUM_WARPS), s>>>(offsets, K, nthreads, buckets, head,
+  launch_after(k_fixup_long<F>, FIX_LONG_BLOCKS, 32 * SUM_WARPS, w_sum_smem<F>(SUM_WARPS), s, offsets, K, nthreads, buckets, head,
                                                                                     tail, hk, err, long_q, long_cap);
   GM_CHECK_LAUNCH("k_fixup_long");
   *launches += 2;
@@ -227,8 +227,8 @@ int reduce_launch(cudaStream_t s, const RedLayout &rl, const xyzz_t<F> *buckets,
   auto *A0 = (xyzz_t<F> *)(ws + rl.o_A0);
   constexpr int WPB = W_THREADS / 32;
   if (rl.warp0) {
-    k_red_level0_warp<F><<<grid_for(rl.G * rl.nseg0, WPB), W_THREADS, w_smem_bytes<F>(WPB), s>>>(
-        buckets, offsets, rl.G, rl.B, rl.L0, rl.nseg0, X, rl.M, A0);
+    launch_after(k_red_level0_warp<F>, grid_for(rl.G * rl.nseg0, WPB), W_THREADS, w_smem_bytes<F>(WPB), s,
+                 buckets, offsets, rl.G, rl.B, rl.L0, rl.nseg0, X, rl.M, A0);
   } else {
     const int64_t wave = (int64_t)rl.sms * level0_blocks_per_sm<F>(rl.dev);
     const int64_t blocks0 = std::min<int64_t>(wave, (rl.G * rl.nseg0 + 127) / 128);
@@ -238,8 +238,8 @@ int reduce_launch(cudaStream_t s, const RedLayout &rl, const xyzz_t<F> *buckets,
   GM_CHECK_LAUNCH("k_red_level0");
   (*launches)++;
   if (rl.nseg1 > 0) {
-    k_red_level1<F><<<grid_for(rl.G * rl.nseg1, WPB), W_THREADS, w_smem_bytes<F>(WPB), s>>>(
-        A0, rl.G, rl.nseg0, rl.L1, rl.nseg1, rl.L0, X, rl.M);
+    launch_after(k_red_level1<F>, grid_for(rl.G * rl.nseg1, WPB), W_THREADS, w_smem_bytes<F>(WPB), s,
+                 A0, rl.G, rl.nseg0, rl.L1, rl.nseg1, rl.L0, X, rl.M);
     GM_CHECK_LAUNCH("k_red_level1");
     (*launches)++;
   }
@@ -248,7 +248,7 @@ int reduce_launch(cudaStream_t s, const RedLayout &rl, const xyzz_t<F> *buckets,
   while (N > 1) {
     const int chunk = RedLayout::sum_chunk(N), nout = (N + chunk - 1) / chunk;
     auto *dst = (xyzz_t<F> *)(ws + rl.o_t[k]);
-    k_red_sum<F><<<(unsigned)(rl.G * nout), 32 * SUM_WARPS, w_sum_smem<F>(SUM_WARPS), s>>>(src, N, chunk, nout, dst);
+    launch_after(k_red_sum<F>, (unsigned)(rl.G * nout), 32 * SUM_WARPS, w_sum_smem<F>(SUM_WARPS), s, src, N, chunk, nout, dst);
     GM_CHECK_LAUNCH("k_red_sum");
     (*launches)++;
     src = dst;
@@ -374,7 +374,7 @@ int msm_run(cudaStream_t s, const MsmLayout<F> &lay, char *ws, const uint4 *base
     handoff->W = W;
     handoff->c = lay.dp.c;
   } else {
-    k_combine<F><<<1, COMBINE_THREADS<F>, combine_smem<F>(), s>>>(src, W, lay.dp.c, nullptr, out,
+    launch_after(k_combine<F>, 1, COMBINE_THREADS<F>, combine_smem<F>(), s, src, W, lay.dp.c, nullptr, out,
                                                                                     affine);
     GM_CHECK_LAUNCH("k_combine");
     launches++;

@@ -281,6 +281,32 @@ GM_DEVI uint32_t block_exclusive_scan(uint32_t v, uint32_t &total) {
   return warp_prefix + x - v;
 }
 
+// Exclusive scan in place of up to SCAN_ONE values, and their sum behind them,
+// in one block: one launch of 3 to 5 us where three take 7.
+constexpr int SCAN_ONE = 4 * SCAN_TILE;
+static __global__ void k_scan_one(uint32_t *__restrict__ a, int n) {
+  uint32_t running = 0;
+  for (int base = 0; base < n; base += SCAN_TILE) {
+    const int i0 = base + threadIdx.x * SCAN_PER_THREAD;
+    uint32_t v[SCAN_PER_THREAD], s = 0;
+#pragma unroll
+    for (int k = 0; k < SCAN_PER_THREAD; k++) {
+      v[k] = (i0 + k < n) ? a[i0 + k] : 0;
+      s += v[k];
+    }
+    uint32_t total;
+    uint32_t ex = block_exclusive_scan(s, total) + running;
+#pragma unroll
+    for (int k = 0; k < SCAN_PER_THREAD; k++) {
+      if (i0 + k < n) a[i0 + k] = ex;
+      ex += v[k];
+    }
+    running += total;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) a[n] = running;
+}
+
 static __global__ void k_scan_blocksum(const uint32_t *__restrict__ in, int64_t K, uint32_t *__restrict__ bsum) {
   const int64_t base = (int64_t)blockIdx.x * SCAN_TILE + threadIdx.x * SCAN_PER_THREAD;
   uint32_t s = 0;
@@ -358,6 +384,39 @@ GM_DEVI int64_t seek_bucket(const uint32_t *__restrict__ offsets, int64_t k, int
   for (int s = 0; s < 4; s++, k++)
     if (__ldg(offsets + k + 1) > pos) return k;
   return k + bucket_of(offsets + k, K - k, pos);
+}
+
+// Programmatic dependent launch: a kernel started with launch_after may begin
+// while the one before it on the stream still runs, and waits in grid_wait
+// before it touches anything that one wrote; what it does before (tables into
+// shared memory, its own launch) costs nothing then.  Every block calls
+// grid_wait first of all, so "the kernel before has ended" holds along the whole
+// stream.  The pointers that are read go through it: a load by the read-only
+// path could be moved over a plain barrier.  grid_release lets the next kernel start.
+template <class P>
+GM_DEVI void grid_opaque(P &p) {
+  asm volatile("" : "+l"(p));
+}
+template <class... P>
+GM_DEVI void grid_wait(P &...p) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  (grid_opaque(p), ...);
+}
+GM_DEVI void grid_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+template <class... P, class... A>
+static inline void launch_after(void (*k)(P...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at = {};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k, P(args)...);
 }
 
 // Asynchronous 16-byte global -> shared copy (cp.async, L2 only).

@@ -52,6 +52,8 @@ __global__ void __launch_bounds__(W_THREADS) k_accumulate_warp(
   using W = WF<F>;
   using E = typename W::E;
   w_setup();
+  grid_wait(bases, entries, offsets);
+  grid_release();
   const int64_t t = (int64_t)blockIdx.x * (W_THREADS / 32) + w_warp();
   if (t >= nslices) return;
   const uint32_t M = __ldg(offsets + K);
@@ -155,6 +157,8 @@ __global__ void __launch_bounds__(W_THREADS) k_red_level0_warp(const xyzz_t<F> *
                                                                int L0, int nseg0, xyzz_t<F> *__restrict__ X, int M,
                                                                xyzz_t<F> *__restrict__ A0) {
   w_setup();
+  grid_wait(buckets, offsets);
+  grid_release();
   const int64_t t = (int64_t)blockIdx.x * (W_THREADS / 32) + w_warp();
   if (t >= G * nseg0) return;
   const int64_t g = t / nseg0;
@@ -175,6 +179,8 @@ template <class F>
 __global__ void __launch_bounds__(W_THREADS) k_red_level1(const xyzz_t<F> *__restrict__ A0, int64_t G, int nseg0,
                                                           int L1, int nseg1, int L0, xyzz_t<F> *__restrict__ X, int M) {
   w_setup();
+  grid_wait(A0);
+  grid_release();
   const int64_t t = (int64_t)blockIdx.x * (W_THREADS / 32) + w_warp();
   if (t >= G * nseg1) return;
   const int64_t g = t / nseg1;
@@ -196,6 +202,8 @@ template <class F>
 __global__ void __launch_bounds__(32 * SUM_WARPS) k_red_sum(const xyzz_t<F> *__restrict__ in, int N, int chunk,
                                                             int nout, xyzz_t<F> *__restrict__ out) {
   w_setup();
+  grid_wait(in);
+  grid_release();
   const int64_t g = blockIdx.x / nout;
   const int i = (int)(blockIdx.x % nout);
   const int j1 = min(N, (i + 1) * chunk);
@@ -227,6 +235,8 @@ __global__ void __launch_bounds__(W_THREADS) k_fixup_split(const uint32_t *__res
                                                            uint32_t *__restrict__ err, int32_t *__restrict__ long_q,
                                                            int64_t long_cap) {
   w_setup();
+  grid_wait(offsets, part_head, part_tail, head_key, tail_key);
+  grid_release();
   const int64_t t = (int64_t)blockIdx.x * (W_THREADS / 32) + w_warp();
   if (t >= nslices) return;
   const int32_t k = __ldg(tail_key + t);
@@ -266,9 +276,11 @@ __global__ void __launch_bounds__(32 * SUM_WARPS) k_fixup_long(const uint32_t *_
                                                                const int32_t *__restrict__ head_key,
                                                                uint32_t *__restrict__ err,
                                                                const int32_t *__restrict__ long_q, int64_t long_cap) {
+  w_setup();
+  grid_wait(offsets, part_head, part_tail, head_key, long_q);
+  grid_release();
   const int64_t n_long = min((int64_t)long_q[0], long_cap);
   if ((int64_t)blockIdx.x >= n_long) return;
-  w_setup();
   const int w = w_warp();
   const uint32_t M = __ldg(offsets + K);
   const uint64_t chunk64 = ((uint64_t)M + nslices - 1) / nslices;
@@ -316,6 +328,8 @@ __global__ void __launch_bounds__(COMBINE_THREADS<F>) k_combine(const xyzz_t<F> 
   using WP = WF<F>;
   constexpr int PT = w_pt_words<F>(), LW = WP::LW;
   w_setup();
+  grid_wait(S);
+  grid_release();
   const int64_t i = blockIdx.x;
   const int w = w_warp();
   constexpr int NCH = Chain<F>::WARPS, LEAD = COMBINE_WARPS;  // the chain's warps are LEAD .. LEAD + NCH - 1

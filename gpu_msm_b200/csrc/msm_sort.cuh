@@ -591,6 +591,11 @@ struct SortLayout {
 // In-place exclusive scan of a[0, len); a[len] receives the total.
 inline void scan_inplace(cudaStream_t s, uint32_t *a, int64_t len, uint32_t *bsum, int *launches) {
   const int64_t nb = SortLayout::scan_blocks(len);
+  if (len <= SCAN_ONE) {
+    k_scan_one<<<1, SCAN_THREADS, 0, s>>>(a, (int)len);
+    *launches += 1;
+    return;
+  }
   k_scan_blocksum<<<(unsigned)nb, SCAN_THREADS, 0, s>>>(a, len, bsum);
   k_scan_top<<<1, SCAN_THREADS, 0, s>>>(bsum, (int)nb);
   k_scan_final<<<(unsigned)nb, SCAN_THREADS, 0, s>>>(a, len, bsum, a);
