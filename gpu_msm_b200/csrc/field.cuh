@@ -600,15 +600,6 @@ struct FpOut : Fp {
   GM_DEVI static fp_t mul(const fp_t &a, const fp_t &b) { return fp_mul_call(a, b); }
   GM_DEVI static fp_t sqr(const fp_t &a) { return fp_sqr_call(a); }
 };
-// The bucket-accumulation loop squares through the general product: with a
-// second ~900-instruction out-of-line function its loop no longer stays in
-// the instruction cache, which costs more than the squaring saves (measured
-// on B200: 13.68 ms against 13.30 ms for the G1 2^20 accumulation).
-struct FpOutMulOnly : Fp {
-  GM_DEVI static fp_t mul(const fp_t &a, const fp_t &b) { return fp_mul_call(a, b); }
-  GM_DEVI static fp_t sqr(const fp_t &a) { return fp_mul_call(a, a); }
-};
-
 // 16-byte vector loads/stores of field elements (56 B = 3.5 x 16 B, so
 // records are laid out with 16-byte alignment by the packers).
 GM_DEVI void load_fp_u64(fp_t &r, const uint64_t *src) {

@@ -55,14 +55,15 @@ struct OutOfLine<Fp2> {
   using type = Fp2Call;
 };
 
-// Policy of the accumulation loop (one out-of-line product only).
+// Policy of the accumulation loop.
 template <class F>
 struct AccPolicy;
-// G1: the integer CIOS product out of line, squares through it too (one
-// product function in the loop).
+// G1: product and square out of line, a square being 1501 cycles a warp
+// where the product is 1855: 65536 points accumulate in 0.87 ms, against 0.92
+// with squares through the product.
 template <>
 struct AccPolicy<Fp> {
-  using type = FpOutMulOnly;
+  using type = FpOut;
 };
 // G2: the whole Fp2 product out of line.  Inlined Karatsuba sums around 30
 // Fp calls made the loop overflow the instruction cache (ncu: 9.9% of warp
