@@ -8,7 +8,7 @@ shard (weak scaling); the shards' partial sums are exchanged with one
 all_gather and added on the device, as a sharded MSM does.
 
 Keys beyond the driver contract:
-  roofline      the dominant kernel (bucket accumulation): its fixed op count
+  roofline      the additions of entries (affine rounds, accumulation): their fixed op count
                 (798 IMAD per Fp product) against the measured mad.lo peak of
                 this GPU (bound "imad": the path is exact integer arithmetic;
                 neither tensor cores nor HBM bound it)
@@ -42,7 +42,7 @@ sys.path.insert(0, ROOT)
 LOG2N = 20
 G2_LOG2N = 18
 # the timed plain-MSM steps run round-robin over this many streams: one MSM's
-# latency-bound tail (upper reduction levels, host window combine) then
+# latency-bound tail (upper reduction levels, window combine) then
 # overlaps the next MSM's accumulation (G1 2^20: 16.6 -> 15.3 ms per MSM)
 PIPELINE_STREAMS = 3
 # CPU baseline sample: the first 2^16 points (about 1 s per pass on 16 host
@@ -188,10 +188,11 @@ class ClockSampler:
 
 
 # ---------------------------------------------------------------------------
-# k_accumulate<Fp> at G1 2^20, from the ncu capture summarised in
-# profiles/k_accumulate_g1_2p20.md: DRAM bytes per launch and pipe utilisation
-ACC_TRAFFIC_NCU = 1.594e9
-ACC_PIPES_NCU = {"fmaheavy_imad": 0.875, "alu": 0.215, "issue": 0.408}
+# Additions of G1 2^20 entries (four k_affine_round<Fp> launches and
+# k_accumulate<Fp>): DRAM bytes of the four rounds and their pipe utilisation,
+# from the ncu capture summarised in profiles/k_affine_round.md
+ADD_TRAFFIC_NCU = 13.95e9
+ADD_PIPES_NCU = {"fmaheavy_imad": 0.725, "alu": 0.237, "issue": 0.347}
 
 # CPU baseline: reference host code (or the oracle port) on a bounded sample
 # ---------------------------------------------------------------------------
@@ -330,7 +331,7 @@ def run_ours(args, rank, world, local_rank):
     def run_steps(steps, pipelined):
         """Device time per step (ms): one stream, or steps round-robin over
         PIPELINE_STREAMS streams (one step's latency-bound tail -- upper
-        reduction levels, host combine -- overlaps the next step's
+        reduction levels, window combine -- overlaps the next step's
         accumulation)."""
         ev0, ev1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
         ev0.record(main)
@@ -371,7 +372,11 @@ def run_ours(args, rank, world, local_rank):
     serial_aff = gm.canonical_affine(gm.to_numpy_proj(outs[0], 1), 1)
 
     # timed region: the same steps, pipelined over PIPELINE_STREAMS streams
-    run_steps(max(args.warmup, PIPELINE_STREAMS), pipelined=True)
+    # (untimed first until every stream's MSM has its workspace: a pass can
+    # find one fewer than it would use, since an allocation that waits lets an
+    # earlier MSM's workspace come free)
+    for _ in range(PIPELINE_STREAMS):
+        run_steps(max(args.warmup, PIPELINE_STREAMS), pipelined=True)
     gm.launch_count_reset()
     if world > 1:
         dist.barrier()
@@ -425,8 +430,12 @@ def run_ours(args, rank, world, local_rank):
     # extra pipe time).
     imad_peak = peaks[1]
 
-    acc_ms = phase_ms.get("accumulate", float("nan"))
-    acc_imad = 798.0 * 10 * entries
+    # additions of entries: affine rounds and the accumulation of what they
+    # leave.  Every entry is counted as one affine addition (6 products with
+    # its share of the inversion); those that the accumulation adds in XYZZ
+    # form take 10, so the rate is a lower bound.
+    acc_ms = phase_ms.get("affine", 0.0) + phase_ms.get("accumulate", float("nan"))
+    acc_imad = 798.0 * 6 * entries
     achieved = acc_imad / (acc_ms / 1e3)
     msm_ops = wl.msm_roofline_imad(n, 1)
 
@@ -441,17 +450,17 @@ def run_ours(args, rank, world, local_rank):
                    "l2": "inputs 168 MB > 126 MB L2 (no flush)"},
         "ms_per_step_serial": serial_ms_max,
         "pipelined_results_equal": bool(pipelined_ok),
-        "roofline": {"bound": "imad", "kernel": "k_accumulate<Fp>", "achieved": achieved / 1e12,
+        "roofline": {"bound": "imad", "kernel": "k_affine_round<Fp> + k_accumulate<Fp>", "achieved": achieved / 1e12,
                      "peak": imad_peak / 1e12, "unit": "TIMAD/s", "frac": achieved / imad_peak,
-                     # dram__bytes_read + dram__bytes_write of one launch, from the ncu
-                     # capture summarised in profiles/k_accumulate_g1_2p20.md
-                     "traffic": ACC_TRAFFIC_NCU,
-                     "traffic_unit": "bytes per launch (ncu)",
-                     "work": f"798 IMAD-equivalents x 10 Fp mults x {entries} entries per launch",
+                     # dram__bytes_read + dram__bytes_write of one MSM's affine rounds,
+                     # from the ncu capture summarised in profiles/k_affine_round.md
+                     "traffic": ADD_TRAFFIC_NCU,
+                     "traffic_unit": "bytes per MSM (ncu, affine rounds)",
+                     "work": f"798 IMAD-equivalents x 6 Fp mults x {entries} entries per MSM",
                      "peak_source": "measured: gm_imad_probe mode 1 (independent mad.lo chains over all SMs)",
                      "peak_lo_hi_mix": peaks[0] / 1e12,
                      "products_on": "IMAD pipe (CIOS, mad.lo.cc/madc.hi.cc)",
-                     "pipes_busy_ncu": ACC_PIPES_NCU},
+                     "pipes_busy_ncu": ADD_PIPES_NCU},
         "msm_roofline": {"ops_imad": msm_ops, "achieved": msm_ops / (ms_max / 1e3) / 1e12,
                          "frac": msm_ops / (ms_max / 1e3) / imad_peak, "unit": "TIMAD/s",
                          "frac_serial": msm_ops / (serial_ms_max / 1e3) / imad_peak},

@@ -9,6 +9,9 @@
 //                  key  key = w*B + |d|-1  (B = 2^(c-1) buckets per window),
 //                  with the bucket offsets (msm_sort.cuh; k_scan_* below are
 //                  its prefix sums).
+//     k_affine_round (MSMs with several points to a bucket, and many) adds the
+//                  points of every bucket in pairs, round by round, so that
+//                  few are left to step 4 (msm_affine.cuh).
 //  4. k_accumulate every thread sums an equal-length slice of the sorted
 //                  entries with XYZZ mixed additions; buckets that fit in a
 //                  slice are written directly, the edge pieces of buckets that
