@@ -11,10 +11,12 @@
 // that are much larger, so those need no rule of their own here.
 //
 // Bound: the multiplier, as for k_accumulate (a round moves 640 bytes an
-// addition, 1.5 TB/s).  B200, G1 2^20 (19.5 M entries, 28 to a bucket): 0.42 ns
-// an addition in the first rounds against 0.55 ns in k_accumulate; accumulation
-// in all 11.1 -> 8.8 ms, G2 2^18 8.7 -> 7.0 ms.  Three blocks of 128 threads
-// per SM (G1): two measured 9.14 ms against 8.79 for six rounds, four 9.00 (the
+// addition, 1.5 TB/s).  B200, G1 2^20 at c = 16 (19.5 M entries, 28 to a
+// bucket): 0.42 ns an addition in the first rounds against 0.55 ns in
+// k_accumulate; accumulation in all 11.1 -> 8.8 ms, G2 2^18 8.7 -> 7.0 ms (at
+// c = 15).  With the widths now chosen (15, 12): 8.0 + 0.8 and 6.4 + 1.4 ms, the
+// multiplier 70-75 % busy in the rounds.  Three blocks of 128 threads per SM
+// (G1): two measured 9.14 ms against 8.79 for six rounds, four 9.00 (the
 // code of product, square, inversion and loops then outgrows the instruction
 // cache).
 //
@@ -41,6 +43,11 @@ constexpr int AFF_MAX_ROUNDS = 8;
 // 4.25, G1 200000 3.41 / 3.34 / 3.46 / 3.46, G2 130000 6.18 / 6.13 / 6.48 / 6.47,
 // G2 65536 4.33 / 4.27 / 4.60 / 4.60 (without rounds: 13.66, 4.56, 3.77, 7.23, 4.60).
 constexpr int AFF_LAST = 16;
+// The two buffers' bytes in all: a chunk's last round and every round's last
+// blocks leave the GPU partly idle, so fewer chunks are better.  Measured with
+// 0.5 / 1 / 3 / 6 / 12 GiB: G1 2^20 12.3 / 11.3 / 10.8 (one chunk), G1 2^21 26.0 /
+// 21.2 / 20.1 / 19.5 / 19.5, G2 2^20 42.0 / 32.2 / 29.2 / 28.9 / 28.9, 512 MSMs of
+// 6 M points 122.6 / 106.9 / 97.3 / 96.6 / 95.7 ms.
 constexpr size_t AFF_SCRATCH = size_t(3) << 30;
 template <class F>
 constexpr int AFF_BLOCKS = sizeof(typename F::T) == sizeof(fp_t) ? 3 : 2;  // resident blocks per SM

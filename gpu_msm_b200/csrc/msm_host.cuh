@@ -125,7 +125,8 @@ struct MsmLayout {
 // k_accumulate runs at most ACC_BLOCKS_MAX blocks per SM.  Its slices carry
 // equal work, so a block that shares its SM with more blocks than the others
 // finishes late and holds up the whole launch: with 3 blocks per SM the G1
-// 2^20 accumulation took 13.8 ms against 13.3 ms, and batches, whose classes'
+// 2^20 accumulation without affine rounds took 13.8 ms against 13.3 ms (with
+// them 3 is slower again), and batches, whose classes'
 // launches overlap, 196 ms against 143 ms.  The grid holds ACC_BLOCKS_MAX
 // blocks per SM, and where the registers would let more blocks share an SM
 // the launch asks for enough dynamic shared memory to keep them out.
