@@ -423,12 +423,14 @@ static inline void launch_after(void (*k)(P...), unsigned grid, unsigned block, 
   cudaLaunchKernelEx(&cfg, k, P(args)...);
 }
 
-// Asynchronous 16-byte global -> shared copy (cp.async, L2 only).
+// Asynchronous 16-byte global -> shared copy (cp.async, L2 only).  It writes
+// shared memory that plain loads read before and after it, so it orders them:
+// a thread's stage slot is read to the end before the next copy overwrites it.
 GM_DEVI void cp_async16(void *smem, const void *gmem) {
   const uint32_t s = (uint32_t)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
 }
-GM_DEVI void cp_async_commit() { asm volatile("cp.async.commit_group;"); }
+GM_DEVI void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 template <int N>
 GM_DEVI void cp_async_wait() {  // all but the N newest groups
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
