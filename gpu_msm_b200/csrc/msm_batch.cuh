@@ -206,16 +206,15 @@ int batch_class_accumulate(const BatchPlan &plan, const BatchClassPlan &cp, cuda
   return GM_OK;
 }
 
-// Enqueue one class's whole pipeline on `s`; rounds: with the affine rounds
-// (not where classes run beside each other: they share the rounds' scratch).
+// Enqueue one class's whole pipeline on `s`.
 template <class F>
-int batch_class_run(const BatchPlan &plan, const BatchClassPlan &cp, cudaStream_t s, bool rounds,
-                    const uint64_t *scalars, uint64_t *results) {
+int batch_class_run(const BatchPlan &plan, const BatchClassPlan &cp, cudaStream_t s, const uint64_t *scalars,
+                    uint64_t *results) {
   if (cp.count == 0) return GM_OK;
   int launches = 0;
   int rc = batch_class_sort<F>(plan, cp, s, scalars, &launches);
   if (rc) return rc;
-  rounds = rounds && plan.rounds(cp);
+  const bool rounds = plan.rounds(cp);
   if (rounds) rc = batch_class_rounds<F>(plan, cp, s, &launches);
   if (rc) return rc;
   rc = batch_class_accumulate<F>(plan, cp, s, rounds, &launches);
@@ -312,6 +311,47 @@ int batch_layouts(BatchPlan &plan, int sms) {
   return GM_OK;
 }
 
+// Every class's pipeline on its own stream, forked from and joined back to s.
+// The classes share the affine rounds' scratch, so those run on s, class after
+// class; the rest of a class with rounds follows them on its stream.  Slices and
+// rounds are those of the queued flow: the results agree word for word.
+template <class F>
+int batch_run_classes(const BatchPlan &plan, cudaStream_t s, const uint64_t *scalars, uint64_t *results) {
+  int launches = 0, rc = GM_OK;
+  GM_CHECK(cudaEventRecord(plan.fork, s));
+  for (const auto &cp : plan.classes) {
+    GM_CHECK(cudaStreamWaitEvent(cp.stream, plan.fork, 0));
+    rc = batch_class_sort<F>(plan, cp, cp.stream, scalars, &launches);
+    if (rc) return rc;
+    if (plan.rounds(cp)) {
+      GM_CHECK(cudaEventRecord(cp.sorted, cp.stream));
+      continue;
+    }
+    rc = batch_class_accumulate<F>(plan, cp, cp.stream, false, &launches);
+    if (rc) return rc;
+    rc = batch_class_finish<F>(plan, cp, cp.stream, false, results, &launches);
+    if (rc) return rc;
+  }
+  for (const auto &cp : plan.classes) {
+    if (!plan.rounds(cp)) continue;
+    GM_CHECK(cudaStreamWaitEvent(s, cp.sorted, 0));
+    rc = batch_class_rounds<F>(plan, cp, s, &launches);
+    if (rc) return rc;
+    GM_CHECK(cudaEventRecord(cp.done, s));
+    GM_CHECK(cudaStreamWaitEvent(cp.stream, cp.done, 0));
+    rc = batch_class_accumulate<F>(plan, cp, cp.stream, true, &launches);
+    if (rc) return rc;
+    rc = batch_class_finish<F>(plan, cp, cp.stream, true, results, &launches);
+    if (rc) return rc;
+  }
+  for (const auto &cp : plan.classes) {
+    GM_CHECK(cudaEventRecord(cp.done, cp.stream));
+    GM_CHECK(cudaStreamWaitEvent(s, cp.done, 0));
+  }
+  count_launches(launches);
+  return GM_OK;
+}
+
 // Fork the classes onto their streams and join them back into `s` (plans
 // with their own streams), or run them in order on `s`.
 template <class F>
@@ -319,21 +359,13 @@ int batch_run(const BatchPlan &plan, cudaStream_t s, const uint64_t *scalars, ui
   if (plan.classes.size() == 1 || plan.fork == nullptr) {
     // one class, or a transient plan without its own streams: in order on s
     for (const auto &cp : plan.classes) {
-      const int rc = batch_class_run<F>(plan, cp, s, true, scalars, results);
+      const int rc = batch_class_run<F>(plan, cp, s, scalars, results);
       if (rc) return rc;
     }
     return GM_OK;
   }
   if (plan.queue && plan.acc_desc) return batch_run_queued<F>(plan, s, scalars, results);
-  GM_CHECK(cudaEventRecord(plan.fork, s));
-  for (const auto &cp : plan.classes) {
-    GM_CHECK(cudaStreamWaitEvent(cp.stream, plan.fork, 0));
-    const int rc = batch_class_run<F>(plan, cp, cp.stream, false, scalars, results);
-    if (rc) return rc;
-    GM_CHECK(cudaEventRecord(cp.done, cp.stream));
-    GM_CHECK(cudaStreamWaitEvent(s, cp.done, 0));
-  }
-  return GM_OK;
+  return batch_run_classes<F>(plan, s, scalars, results);
 }
 
 }  // namespace gm
