@@ -59,7 +59,7 @@ C_API = [
     "gm_g1_msm_device_affine", "gm_g2_msm_device_affine",
     "gm_g1_to_montgomery_batch", "gm_g2_to_montgomery_batch",
     "gm_g1_generator_mul_batch", "gm_g2_generator_mul_batch", "gm_last_error",
-    "gm_profile_enable", "gm_profile_collect", "gm_launch_count_reset", "gm_imad_probe",
+    "gm_trim_memory", "gm_profile_enable", "gm_profile_collect", "gm_launch_count_reset", "gm_imad_probe",
     "gm_g1_sum_projective", "gm_g2_sum_projective", "gm_g1_msm_device_noalloc",
     "gm_bases_create", "gm_bases_destroy", "gm_bases_count", "gm_bases_precompute", "gm_msm_resident", "gm_batch_plan_create",
     "gm_batch_plan_run", "gm_batch_plan_destroy", "gm_batch_plan_bytes", "gm_batch_plan_classes",
@@ -564,6 +564,12 @@ def to_numpy_proj(t, group: int = 1) -> np.ndarray:
     arr = t.detach().cpu().numpy().view(np.uint64)
     pdt = G1P if group == 1 else G2P
     return np.ascontiguousarray(arr).view(pdt).reshape(-1)
+
+
+def trim_memory(device: int = 0):
+    """Give the device memory that the library keeps between calls back to the
+    device (``gm_trim_memory``); waits for the device."""
+    _check(lib().gm_trim_memory(int(device)), "gm_trim_memory")
 
 
 # ---------------------------------------------------------------------------

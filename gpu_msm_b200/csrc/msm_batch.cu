@@ -473,18 +473,18 @@ static int batch_run_once(gm_stream_t stream, const gm_bases *b, int scalar_limb
     off_ws[k] = total;
     total += (plan.classes[k].ws_bytes + 255) / 256 * 256;
   }
-  // the affine rounds' memory behind it, where there is room for it
+  // what the affine rounds leave behind it, where there is room for it; then, in a caller's workspace, their scratch
   std::vector<size_t> off_aff(plan.classes.size());
   size_t with_rounds = total;
   for (size_t k = 0; k < plan.classes.size(); k++) {
     off_aff[k] = with_rounds;
     with_rounds += (plan.classes[k].al.bytes + 255) / 256 * 256;
   }
-  const size_t off_scratch = with_rounds;
-  with_rounds += plan.aff_scratch_bytes();
   bool rounds = with_rounds > total;
   char *mem = nullptr;
   if (ws) {
+    const size_t off_scratch = with_rounds;
+    with_rounds += plan.aff_scratch_bytes();
     if (total > ws_bytes || (size_t)transient_bytes(plan, d64, idx) > ws_bytes ||
         (reinterpret_cast<uintptr_t>(ws) & 255u)) {
       gm::set_last_error("batch workspace too small or not 256-byte aligned");
@@ -492,6 +492,7 @@ static int batch_run_once(gm_stream_t stream, const gm_bases *b, int scalar_limb
     }
     mem = static_cast<char *>(ws);
     rounds = rounds && with_rounds <= ws_bytes;
+    if (rounds) plan.aff_scratch = mem + off_scratch;
   } else {
     rc = rounds ? gm::pool_alloc(plan.dev, s, with_rounds, (void **)&mem) : gm::GM_ERR_ALLOC;
     if (rc) {
@@ -500,8 +501,8 @@ static int batch_run_once(gm_stream_t stream, const gm_bases *b, int scalar_limb
       rc = gm::pool_alloc(plan.dev, s, total, (void **)&mem);
     }
     if (rc) return rc;
+    plan.lease = rounds;
   }
-  if (rounds) plan.aff_scratch = mem + off_scratch;
   // descriptors go through one pinned slot (an asynchronous copy from pageable
   // memory would first wait for the stream), released in stream order
   void *slot = nullptr;
@@ -564,6 +565,11 @@ int gm_batch_plan_destroy(gm_batch_plan *p) {
   cudaDeviceSynchronize();
   free_plan(p);
   return gm::GM_OK;
+}
+
+int gm_trim_memory(uint32_t gpu_index) {
+  const int rc = gm::select_device(gpu_index);
+  return rc ? rc : gm::trim_memory((int)gpu_index);
 }
 
 int64_t gm_batch_plan_bytes(const gm_batch_plan *p) { return p ? (int64_t)p->plan.bytes : 0; }

@@ -55,13 +55,15 @@ struct BatchPlan {
   std::vector<BatchClassPlan> classes;
   cudaEvent_t fork = nullptr;
   size_t bytes = 0;
-  char *aff_scratch = nullptr;  // scratch of the affine rounds, which run class after class (owned)
+  // scratch of the affine rounds, which run class after class: owned, or (lease) a scratch block for each class
+  char *aff_scratch = nullptr;
+  bool lease = false;
   size_t aff_scratch_bytes() const {
     size_t b = 0;
     for (const auto &cp : classes) b = std::max(b, cp.al.scratch);
     return b;
   }
-  bool rounds(const BatchClassPlan &cp) const { return cp.al.rounds > 0 && cp.aff_ws && aff_scratch; }
+  bool rounds(const BatchClassPlan &cp) const { return cp.al.rounds > 0 && cp.aff_ws && (aff_scratch || lease); }
   // Accumulation mode of plans: true (default) = every class's accumulation
   // in one persistent launch over a device work queue (k_accumulate_queue)
   // between the classes' sorts and their fix-ups; false = one pipeline per
@@ -186,12 +188,17 @@ int batch_class_finish(const BatchPlan &plan, const BatchClassPlan &cp, cudaStre
   return GM_OK;
 }
 
-// One class, the affine rounds over its sorted entries.
+// One class, the affine rounds over its sorted entries.  *ran: false where no
+// scratch block could be had (never with the plan's own scratch).
 template <class F>
-int batch_class_rounds(const BatchPlan &plan, const BatchClassPlan &cp, cudaStream_t s, int *launches) {
+int batch_class_rounds(const BatchPlan &plan, const BatchClassPlan &cp, cudaStream_t s, int *launches, bool *ran) {
   ClassBufs<F> cb(plan, cp, false);
-  const cudaError_t e = aff_launch<F>(s, cp.al, cp.aff_ws, plan.aff_scratch, cb.acc_bases, cb.acc_entries,
-                                      cb.acc_offsets, launches);
+  ScratchLease lease;
+  char *scratch = plan.aff_scratch ? plan.aff_scratch : lease.acquire(plan.dev, s, cp.al.scratch);
+  *ran = scratch != nullptr;
+  if (!scratch) return GM_OK;
+  const cudaError_t e = aff_launch<F>(s, cp.al, cp.aff_ws, scratch, cb.acc_bases, cb.acc_entries, cb.acc_offsets,
+                                      launches);
   return e == cudaSuccess ? GM_OK : record_error(e, "k_affine_round");
 }
 
@@ -214,8 +221,8 @@ int batch_class_run(const BatchPlan &plan, const BatchClassPlan &cp, cudaStream_
   int launches = 0;
   int rc = batch_class_sort<F>(plan, cp, s, scalars, &launches);
   if (rc) return rc;
-  const bool rounds = plan.rounds(cp);
-  if (rounds) rc = batch_class_rounds<F>(plan, cp, s, &launches);
+  bool rounds = plan.rounds(cp);
+  if (rounds) rc = batch_class_rounds<F>(plan, cp, s, &launches, &rounds);
   if (rc) return rc;
   rc = batch_class_accumulate<F>(plan, cp, s, rounds, &launches);
   if (rc) return rc;
@@ -268,9 +275,10 @@ int batch_run_queued(const BatchPlan &plan, cudaStream_t s, const uint64_t *scal
     return GM_OK;
   }
   int rc = GM_OK;
+  bool ran = false;
   for (const auto &cp : plan.classes)
     if (plan.rounds(cp)) {
-      rc = batch_class_rounds<F>(plan, cp, s, &launches);
+      rc = batch_class_rounds<F>(plan, cp, s, &launches, &ran);
       if (rc) return rc;
     }
   GM_CHECK(cudaMemsetAsync(plan.queue_ctr, 0, sizeof(uint32_t), s));
@@ -318,6 +326,7 @@ int batch_layouts(BatchPlan &plan, int sms) {
 template <class F>
 int batch_run_classes(const BatchPlan &plan, cudaStream_t s, const uint64_t *scalars, uint64_t *results) {
   int launches = 0, rc = GM_OK;
+  bool ran = false;
   GM_CHECK(cudaEventRecord(plan.fork, s));
   for (const auto &cp : plan.classes) {
     GM_CHECK(cudaStreamWaitEvent(cp.stream, plan.fork, 0));
@@ -335,7 +344,7 @@ int batch_run_classes(const BatchPlan &plan, cudaStream_t s, const uint64_t *sca
   for (const auto &cp : plan.classes) {
     if (!plan.rounds(cp)) continue;
     GM_CHECK(cudaStreamWaitEvent(s, cp.sorted, 0));
-    rc = batch_class_rounds<F>(plan, cp, s, &launches);
+    rc = batch_class_rounds<F>(plan, cp, s, &launches, &ran);
     if (rc) return rc;
     GM_CHECK(cudaEventRecord(cp.done, s));
     GM_CHECK(cudaStreamWaitEvent(cp.stream, cp.done, 0));

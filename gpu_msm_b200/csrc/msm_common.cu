@@ -256,6 +256,136 @@ int pool_alloc(int dev, cudaStream_t s, size_t bytes, void **ptr) {
 }
 
 // ---------------------------------------------------------------------------
+// scratch blocks (msm_engine.h)
+// ---------------------------------------------------------------------------
+struct ScratchBlock {
+  char *p = nullptr;
+  size_t bytes = 0;
+  cudaEvent_t done = nullptr;  // after the block's last use
+  cudaStream_t last = nullptr;
+  uint64_t turn = 0;  // of the last use
+};
+struct ScratchArena {
+  std::mutex mu;
+  ScratchBlock blocks[SCRATCH_BLOCKS];
+  uint64_t turns = 0;
+};
+
+static ScratchArena &scratch_arena(int dev) {
+  static std::mutex mu;
+  static std::map<int, ScratchArena> arenas;  // nodes stay where they are
+  std::lock_guard<std::mutex> lk(mu);
+  return arenas[dev];
+}
+
+bool device_room(size_t bytes) {
+  // also while this thread captures a stream, whose work the question is no part of
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  size_t free_bytes = 0, all = 0;
+  const cudaError_t e = cudaMemGetInfo(&free_bytes, &all);
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e == cudaSuccess) return free_bytes / 2 >= bytes;
+  cudaGetLastError();
+  return false;
+}
+
+static void scratch_drop(ScratchBlock &b) {
+  if (b.p == nullptr) return;
+  cudaEventSynchronize(b.done);
+  cudaFree(b.p);
+  cudaEventDestroy(b.done);
+  b = ScratchBlock();
+}
+
+static bool scratch_create(ScratchBlock &b, size_t bytes) {
+  // four sizes from one power of two to the next: calls of slightly different sizes share a block
+  size_t step = size_t(16) << 20;
+  while (8 * step < bytes) step *= 2;
+  const size_t up = (bytes + step - 1) / step * step;
+  if (!device_room(up)) return false;
+  if (cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming) == cudaSuccess) {
+    if (cudaMalloc(&b.p, up) == cudaSuccess) {
+      b.bytes = up;
+      return true;
+    }
+    cudaEventDestroy(b.done);
+  }
+  cudaGetLastError();
+  b = ScratchBlock();
+  return false;
+}
+
+char *ScratchLease::acquire(int dev, cudaStream_t s, size_t bytes) {
+  release();
+  dev_ = dev;
+  s_ = s;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    void *p = nullptr;
+    if (!device_room(bytes) || pool_alloc(dev, s, bytes, &p) != GM_OK) {
+      cudaGetLastError();
+      return nullptr;
+    }
+    return captured_ = static_cast<char *>(p);
+  }
+  ScratchArena &a = scratch_arena(dev);
+  std::unique_lock<std::mutex> lk(a.mu);
+  // the stream's own last block, an idle one, a new one, the one in use for longest, a new one in place of a smaller
+  ScratchBlock *own = nullptr, *idle = nullptr, *used = nullptr, *empty = nullptr, *small = nullptr;
+  for (ScratchBlock &b : a.blocks) {
+    if (b.p == nullptr) {
+      empty = &b;
+    } else if (b.bytes < bytes) {
+      if ((!small || b.bytes < small->bytes) && cudaEventQuery(b.done) == cudaSuccess) small = &b;
+    } else if (b.last == s) {
+      own = &b;
+    } else if (cudaEventQuery(b.done) == cudaSuccess) {
+      idle = &b;
+    } else if (!used || b.turn < used->turn) {
+      used = &b;
+    }
+  }
+  ScratchBlock *take = own ? own : idle;
+  if (!take && empty && scratch_create(*empty, bytes)) take = empty;
+  if (!take) take = used;
+  if (!take && small) {
+    scratch_drop(*small);
+    if (scratch_create(*small, bytes)) take = small;
+  }
+  cudaGetLastError();  // a query's "not ready"
+  if (!take || cudaStreamWaitEvent(s, take->done, 0) != cudaSuccess) return nullptr;
+  take->last = s;
+  take->turn = ++a.turns;
+  lk.release();  // until release()
+  block_ = take;
+  return take->p;
+}
+
+void ScratchLease::release() {
+  if (captured_) cudaFreeAsync(captured_, s_);
+  captured_ = nullptr;
+  if (!block_) return;
+  if (cudaEventRecord(block_->done, s_) != cudaSuccess) cudaStreamSynchronize(s_);
+  block_ = nullptr;
+  scratch_arena(dev_).mu.unlock();
+}
+
+int trim_memory(int dev) {
+  GM_CHECK(cudaDeviceSynchronize());
+  {
+    ScratchArena &a = scratch_arena(dev);
+    std::lock_guard<std::mutex> lk(a.mu);
+    for (ScratchBlock &b : a.blocks) scratch_drop(b);
+  }
+  DeviceState *st;
+  const int rc = device_state(dev, &st);
+  if (rc) return rc;
+  GM_CHECK(cudaMemPoolTrimTo(st->pool, 0));
+  return GM_OK;
+}
+
+// ---------------------------------------------------------------------------
 // window selection (cost model in multiplication units)
 //   accumulation: 10 per (point, non-zero window) (madd 8M+2S), 7 where rounds
 //                 of affine additions run first (about 3 M entries up)

@@ -42,6 +42,44 @@ int64_t launches_and_reset();
 int pool_alloc(int dev, cudaStream_t s, size_t bytes, void **ptr);
 int default_window(int group, int64_t n, int limbs);
 
+// Device memory that one call's kernels use for a part of their run and that
+// later calls, on any stream, take over: the scratch of the affine rounds.
+//
+// A device keeps up to SCRATCH_BLOCKS blocks.  acquire orders the stream after
+// the block's last use and holds it for the calling thread, which enqueues its
+// kernels and then calls release; the host waits only while another thread
+// enqueues.  A call takes a block that is idle or was last used on its own
+// stream, or a new one; only with SCRATCH_BLOCKS calls in flight does it take
+// its turn behind one of them, so that the memory kept is bounded whatever the
+// number of streams.  (The rounds fill the GPU: three streams of G1 2^20 points
+// take 10.1 ms a call with three blocks and with one.)  A block comes from cudaMalloc:
+// 3 GB take 0.8 ms where a stream-ordered pool maps them in 18 ms, which a
+// process's first call at a size would pay (B200, first G1 2^20 call 31 to 37 ->
+// 17 ms).  While s is being captured the memory is a graph allocation of its
+// own.  acquire returns null, and the caller does without, where the device
+// does not have twice the bytes free.
+constexpr int SCRATCH_BLOCKS = 4;
+struct ScratchBlock;
+class ScratchLease {
+ public:
+  ScratchLease() = default;
+  ScratchLease(const ScratchLease &) = delete;
+  ScratchLease &operator=(const ScratchLease &) = delete;
+  ~ScratchLease() { release(); }
+  char *acquire(int dev, cudaStream_t s, size_t bytes);
+  void release();
+
+ private:
+  int dev_ = 0;
+  cudaStream_t s_ = nullptr;
+  char *captured_ = nullptr;       // graph allocation
+  ScratchBlock *block_ = nullptr;  // held, with its device's lock
+};
+// Whether the device has twice these bytes free.
+bool device_room(size_t bytes);
+// Gives the kept blocks and the pool's unused memory back to the device.
+int trim_memory(int dev);
+
 // Window sums handed to a synchronous caller in place of the device
 // combination: the MSM copies its W window sums (XYZZ, device layout) to
 // `host` (pinned, `cap` bytes), sets W and c and writes no result; the caller

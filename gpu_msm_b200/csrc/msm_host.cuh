@@ -80,8 +80,8 @@ struct MsmLayout {
   int64_t long_cap = 0;
   bool need_pack = false;
   bool warp_acc = false;  // accumulation slices on warps
-  AffLayout al;
-  size_t o_aff = 0, o_aff_scratch = 0;
+  AffLayout al;  // its scratch is not part of the workspace (ScratchLease)
+  size_t o_aff = 0;
   SortLayout sl;
   RedLayout rl;
 
@@ -116,7 +116,6 @@ struct MsmLayout {
     o_err = cv.take<uint32_t>(4);
     if (affine_rounds) al.plan<F, Carve>(&n, 1, dp.W, 1, dp.B, sms);
     o_aff = cv.take<char>(al.bytes);
-    o_aff_scratch = cv.take<char>(al.scratch);
     o_packed = pack ? cv.take<uint4>((size_t)n * Rec<F>::U4) : 0;
     bytes = cv.off;
   }
@@ -290,7 +289,8 @@ int msm_plan(MsmLayout<F> &lay, int dev, int64_t n, int limbs, int c, bool pack,
 }
 
 // Enqueues the whole pipeline of one planned MSM on s, in the workspace ws
-// (lay.bytes, 256-byte aligned); allocates nothing itself.  bases: packed
+// (lay.bytes, 256-byte aligned); allocates nothing itself, except that the
+// affine rounds, where planned, run in a scratch block if the device has room for one.  bases: packed
 // records, or null to pack from ref_points (reference layout; to_mont converts
 // standard-form points).  out receives the result in the reference layout,
 // projective or (affine) affine.  err_out (optional,
@@ -337,12 +337,15 @@ int msm_run(cudaStream_t s, const MsmLayout<F> &lay, char *ws, const uint4 *base
     profile_mark(s, "pack");
   }
   if (lay.al.rounds > 0) {
-    const cudaError_t e = aff_launch<F>(s, lay.al, ws + lay.o_aff, ws + lay.o_aff_scratch, bases, entries, offsets, &launches);
-    if (e != cudaSuccess) return record_error(e, "k_affine_round");
-    profile_mark(s, "affine");
-    bases = lay.al.final_points(ws + lay.o_aff);
-    entries = nullptr;
-    offsets = lay.al.final_offsets(ws + lay.o_aff);
+    ScratchLease lease;
+    if (char *scratch = lease.acquire(lay.rl.dev, s, lay.al.scratch)) {
+      const cudaError_t e = aff_launch<F>(s, lay.al, ws + lay.o_aff, scratch, bases, entries, offsets, &launches);
+      if (e != cudaSuccess) return record_error(e, "k_affine_round");
+      profile_mark(s, "affine");
+      bases = lay.al.final_points(ws + lay.o_aff);
+      entries = nullptr;
+      offsets = lay.al.final_offsets(ws + lay.o_aff);
+    }
   }
   acc_launch<F>(lay.warp_acc, s, bases, entries, offsets, lay.K, lay.nthreads, buckets, head, tail, hk, tk);
   GM_CHECK_LAUNCH("k_accumulate");
@@ -401,7 +404,7 @@ int msm_launch(cudaStream_t s, int dev, const uint4 *bases, const uint64_t *ref_
     return GM_OK;
   }
   const int c = c_override > 0 ? c_override : default_window(sizeof(typename F::T) == sizeof(fp_t) ? 1 : 2, n, limbs);
-  // without the affine rounds where the device has no room for their scratch
+  // without the affine rounds where the device has no room for what they leave
   MsmLayout<F> lay;
   char *ws = nullptr;
   int rc = GM_OK;

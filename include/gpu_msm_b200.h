@@ -96,6 +96,14 @@ int g1_msm_limbs_wrapper(G1ProjectivePoint *result, const G1Point *points, const
 int g2_msm_limbs_wrapper(G2ProjectivePoint *result, const G2Point *points, const uint64_t *scalars,
                          int scalar_limbs, int n, uint32_t gpu_index, int points_montgomery);
 
+/* Gives the device memory that the library keeps between calls back to the
+ * device: the unused part of the stream-ordered pool that workspaces come
+ * from, and the scratch blocks of large MSMs: one per call in flight (0.5 to
+ * 3.5 GiB, 7 GiB after single MSMs of 2^25 points), at most four, which calls on
+ * further streams take in turn.  Waits for the device.  Later calls take memory
+ * again.  No reference counterpart (its callers own the scratch buffers). */
+int gm_trim_memory(uint32_t gpu_index);
+
 /* Host-buffer MSM, asynchronous on `stream`: the same computation as
  * g{1,2}_msm_limbs_wrapper, enqueued instead of waited for.  The scalar and
  * point copies from host memory, the MSM and the copy of the projective

@@ -1,0 +1,136 @@
+"""GPU: the scratch blocks of the rounds of affine additions: shared by streams
+and threads, bounded, given back, replaced by a graph's own memory under
+capture, and done without where the device has no room.  Results agree word
+for word wherever the rounds run."""
+import threading
+
+import numpy as np
+import pytest
+import torch
+
+import gpu_msm_b200 as gm
+import oracle
+from gpu_msm_b200 import workload as wl
+
+pytestmark = pytest.mark.gpu
+N, C = 131072, 10  # 4.3 M entries, two rounds: 0.65 GB of scratch, 0.25 GB of workspace
+
+
+def dev(a, cuda):
+    return torch.from_numpy(np.ascontiguousarray(a).view(np.int64)).to(cuda)
+
+
+@pytest.fixture(scope="module")
+def case():
+    cuda = torch.device("cuda:0")
+    logs, sc = wl.make_base_logs(N, seed=61), wl.make_scalars(N, seed=62)
+    pts, scd = gm.generator_mul_batch(dev(logs, cuda)), dev(sc, cuda)
+    out = gm.msm_device(pts, scd, window_bits=C)
+    torch.cuda.synchronize()
+    got = oracle.proj_to_affine(gm.to_numpy_proj(out))
+    assert oracle.same_point(got, oracle.generator_multiple(wl.expected_log(sc, logs)))
+    return pts, scd, out
+
+
+def free():
+    torch.cuda.synchronize()
+    return torch.cuda.mem_get_info()[0]
+
+
+def phases(pts, sc):
+    gm.profile_enable(True)
+    try:
+        out = gm.msm_device(pts, sc, window_bits=C)
+        return [name for name, _ in gm.profile_collect()], out
+    finally:
+        gm.profile_enable(False)
+
+
+def test_streams_share_and_give_back(case):
+    pts, sc, want = case
+    streams = [torch.cuda.Stream() for _ in range(12)]
+    outs = [torch.empty_like(want) for _ in streams]
+    gm.trim_memory()
+    start = free()
+    gm.msm_device(pts, sc, window_bits=C, out=outs[0], stream=streams[0])
+    one = start - free()
+    for _ in range(3):
+        for s, o in zip(streams, outs):
+            o.zero_()
+        torch.cuda.synchronize()
+        for s, o in zip(streams, outs):
+            gm.msm_device(pts, sc, window_bits=C, out=o, stream=s)
+        torch.cuda.synchronize()
+        assert all(torch.equal(o, want) for o in outs)
+    assert start - free() < 0.6 * len(streams) * one
+    gm.trim_memory()
+    assert start - free() < one / 4
+
+
+def test_threads(case):
+    pts, sc, want = case
+    outs = [[torch.empty_like(want) for _ in range(6)] for _ in range(5)]
+    streams = [torch.cuda.Stream() for _ in outs]
+    torch.cuda.synchronize()
+    errors = []
+
+    def work(s, os):
+        try:
+            for o in os:
+                gm.msm_device(pts, sc, window_bits=C, out=o, stream=s)
+        except Exception as e:  # noqa: BLE001
+            errors.append(e)
+    ts = [threading.Thread(target=work, args=a) for a in zip(streams, outs)]
+    [t.start() for t in ts]
+    [t.join() for t in ts]
+    torch.cuda.synchronize()
+    assert not errors
+    assert all(torch.equal(o, want) for os in outs for o in os)
+
+
+def test_larger_calls_replace_blocks(case):
+    """Blocks too small for the next call; the smaller calls then share the larger block."""
+    pts, sc, want = case
+    gm.trim_memory()
+    streams = [torch.cuda.Stream() for _ in range(5)]
+    small = 60000  # 2 M entries: one round
+    first = gm.msm_device(pts[:small], sc[:small], window_bits=C)
+    torch.cuda.synchronize()
+    for n, ref in ((small, first), (N, want), (small, first), (N, want)):
+        outs = [gm.msm_device(pts[:n], sc[:n], window_bits=C, stream=s) for s in streams]
+        torch.cuda.synchronize()
+        assert all(torch.equal(o, ref) for o in outs), n
+
+
+def test_capture(case):
+    pts, sc, want = case
+    out = torch.empty_like(want)
+    static = sc.clone()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, capture_error_mode="thread_local"):
+        gm.msm_device(pts, static, window_bits=C, out=out)
+    for _ in range(2):
+        out.zero_()
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
+    del g
+
+
+def test_without_room(case):
+    """Room for the workspace, not for twice the scratch: exact without the rounds, and with them again after."""
+    pts, sc, want = case
+    gm.trim_memory()
+    torch.cuda.empty_cache()
+    names, out = phases(pts, sc)
+    assert "affine" in names and torch.equal(out, want)
+    gm.trim_memory()
+    fill = torch.empty(free() - (1400 << 20), dtype=torch.uint8, device=pts.device)
+    names, out = phases(pts, sc)
+    del fill
+    torch.cuda.empty_cache()
+    assert "affine" not in names and "accumulate" in names
+    same = oracle.proj_to_affine(gm.to_numpy_proj(out))
+    assert oracle.same_point(same, oracle.proj_to_affine(gm.to_numpy_proj(want)))
+    names, out = phases(pts, sc)
+    assert "affine" in names and torch.equal(out, want)
