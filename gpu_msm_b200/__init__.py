@@ -59,7 +59,7 @@ C_API = [
     "gm_g1_msm_device_affine", "gm_g2_msm_device_affine",
     "gm_g1_to_montgomery_batch", "gm_g2_to_montgomery_batch",
     "gm_g1_generator_mul_batch", "gm_g2_generator_mul_batch", "gm_last_error",
-    "gm_trim_memory", "gm_profile_enable", "gm_profile_collect", "gm_launch_count_reset", "gm_imad_probe",
+    "gm_trim_memory", "gm_batch_workspace_min_bytes", "gm_profile_enable", "gm_profile_collect", "gm_launch_count_reset", "gm_imad_probe",
     "gm_g1_sum_projective", "gm_g2_sum_projective", "gm_g1_msm_device_noalloc",
     "gm_bases_create", "gm_bases_destroy", "gm_bases_count", "gm_bases_precompute", "gm_msm_resident", "gm_batch_plan_create",
     "gm_batch_plan_run", "gm_batch_plan_destroy", "gm_batch_plan_bytes", "gm_batch_plan_classes",
@@ -130,8 +130,9 @@ def lib() -> ctypes.CDLL:
         L.gm_batch_run.argtypes = [vp, vp, i32, i32, vp, vp, vp, vp, vp]
         L.gm_batch_run_ws.argtypes = [vp, vp, i32, i32, vp, vp, vp, vp, vp, vp, i64]
         L.gm_g1_sum_projective_host.argtypes = [vp, vp, i32]
-        L.gm_batch_workspace_bytes.argtypes = [vp, i32, i32, vp, vp]
-        L.gm_batch_workspace_bytes.restype = i64
+        for name in ("gm_batch_workspace_bytes", "gm_batch_workspace_min_bytes"):
+            getattr(L, name).argtypes = [vp, i32, i32, vp, vp]
+            getattr(L, name).restype = i64
         for name in ("gm_g1_sum_projective", "gm_g2_sum_projective"):
             getattr(L, name).argtypes = [vp, u32, vp, vp, i32]
         for name in ("gm_fp_elem", "gm_fp2_elem"):
@@ -808,8 +809,9 @@ def batch_run(bases: ResidentBases, sizes, scalars, base_offsets=None, window_bi
     """One batch without a plan (``gm_batch_run``): classes in order on the
     stream, for batches whose shape changes on every call.  workspace: None
     takes the device memory from the library's stream-ordered pool for this
-    run; or a uint8 device tensor of at least ``batch_workspace_bytes`` bytes
-    (``gm_batch_run_ws``), in use until the stream has run the batch."""
+    run; or a uint8 device tensor (``gm_batch_run_ws``), in use until the stream
+    has run the batch: ``batch_workspace_bytes`` bytes for the same run as
+    without one, ``batch_workspace_min_bytes`` at the least."""
     import torch
     sizes = np.ascontiguousarray(sizes, dtype=np.int64)
     total = int(sizes.sum())
@@ -835,11 +837,22 @@ def batch_run(bases: ResidentBases, sizes, scalars, base_offsets=None, window_bi
 
 
 def batch_workspace_bytes(bases: ResidentBases, sizes, window_bits=None, scalar_limbs: int = 5) -> int:
+    """Device bytes ``batch_run`` takes for the batch."""
+    return _workspace_bytes("gm_batch_workspace_bytes", bases, sizes, window_bits, scalar_limbs)
+
+
+def batch_workspace_min_bytes(bases: ResidentBases, sizes, window_bits=None, scalar_limbs: int = 5) -> int:
+    """The smallest workspace ``batch_run`` accepts for the batch; a large one
+    runs without the rounds of affine additions in it, and longer."""
+    return _workspace_bytes("gm_batch_workspace_min_bytes", bases, sizes, window_bits, scalar_limbs)
+
+
+def _workspace_bytes(name, bases, sizes, window_bits, scalar_limbs) -> int:
     sizes = np.ascontiguousarray(sizes, dtype=np.int64)
     if window_bits is None:
         window_bits = bases.windows_for(sizes, scalar_limbs)
     wins = np.ascontiguousarray(window_bits, dtype=np.int32)
-    v = int(lib().gm_batch_workspace_bytes(bases.handle, scalar_limbs, len(sizes), _p(sizes), _p(wins)))
+    v = int(getattr(lib(), name)(bases.handle, scalar_limbs, len(sizes), _p(sizes), _p(wins)))
     if v < 0:
-        raise MSMError("gm_batch_workspace_bytes: bad batch")
+        raise MSMError(f"{name}: bad batch")
     return v

@@ -257,16 +257,28 @@ int build_classes(const gm_bases *b, int scalar_limbs, int count, const int64_t 
 
 }  // namespace
 
-// Device bytes of a transient batch (descriptors and workspaces of every
-// class, each 256-byte aligned): the figure gm_batch_workspace_bytes reports
-// and gm_batch_run_ws requires.
+// Device bytes of a transient batch: descriptors and workspaces of every class,
+// each 256-byte aligned; rounds: and what the affine rounds take (the points they
+// leave, and the scratch that they share).
 static int64_t transient_bytes(const gm::BatchPlan &plan, const std::vector<std::vector<int64_t>> &d64,
-                               const std::vector<std::vector<int32_t>> &idx) {
-  int64_t bytes = 0;
-  for (size_t k = 0; k < plan.classes.size(); k++)
-    bytes += (int64_t)(plan.classes[k].ws_bytes + d64[k].size() * sizeof(int64_t) + idx[k].size() * sizeof(int32_t) +
-                       512);
-  return bytes;
+                               const std::vector<std::vector<int32_t>> &idx, bool rounds) {
+  size_t bytes = 0;
+  for (size_t k = 0; k < plan.classes.size(); k++) {
+    bytes += plan.classes[k].ws_bytes + d64[k].size() * sizeof(int64_t) + idx[k].size() * sizeof(int32_t) + 512;
+    if (rounds) bytes += (plan.classes[k].al.bytes + 255) / 256 * 256;
+  }
+  const size_t scratch = plan.aff_scratch_bytes();
+  if (rounds && scratch) bytes += gm::scratch_block_bytes(scratch);
+  return (int64_t)bytes;
+}
+
+static int64_t workspace_bytes(const gm_bases *b, int scalar_limbs, int count, const int64_t *sizes,
+                               const int32_t *window_bits, bool rounds) {
+  gm::BatchPlan plan;
+  std::vector<std::vector<int64_t>> d64;
+  std::vector<std::vector<int32_t>> idx;
+  if (build_classes(b, scalar_limbs, count, sizes, nullptr, window_bits, plan, d64, idx)) return -1;
+  return transient_bytes(plan, d64, idx, rounds);
 }
 
 extern "C" {
@@ -441,11 +453,12 @@ int gm_batch_plan_set_queue(gm_batch_plan *p, int on) {
 
 int64_t gm_batch_workspace_bytes(const gm_bases *b, int scalar_limbs, int count, const int64_t *sizes,
                                  const int32_t *window_bits) {
-  gm::BatchPlan plan;
-  std::vector<std::vector<int64_t>> d64;
-  std::vector<std::vector<int32_t>> idx;
-  if (build_classes(b, scalar_limbs, count, sizes, nullptr, window_bits, plan, d64, idx)) return -1;
-  return transient_bytes(plan, d64, idx);
+  return workspace_bytes(b, scalar_limbs, count, sizes, window_bits, true);
+}
+
+int64_t gm_batch_workspace_min_bytes(const gm_bases *b, int scalar_limbs, int count, const int64_t *sizes,
+                                     const int32_t *window_bits) {
+  return workspace_bytes(b, scalar_limbs, count, sizes, window_bits, false);
 }
 
 // gm_batch_run / gm_batch_run_ws: ws == nullptr takes the workspace from the
@@ -485,7 +498,7 @@ static int batch_run_once(gm_stream_t stream, const gm_bases *b, int scalar_limb
   if (ws) {
     const size_t off_scratch = with_rounds;
     with_rounds += plan.aff_scratch_bytes();
-    if (total > ws_bytes || (size_t)transient_bytes(plan, d64, idx) > ws_bytes ||
+    if (total > ws_bytes || (size_t)transient_bytes(plan, d64, idx, false) > ws_bytes ||
         (reinterpret_cast<uintptr_t>(ws) & 255u)) {
       gm::set_last_error("batch workspace too small or not 256-byte aligned");
       return gm::GM_ERR_ARG;

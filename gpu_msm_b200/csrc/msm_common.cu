@@ -298,11 +298,15 @@ static void scratch_drop(ScratchBlock &b) {
   b = ScratchBlock();
 }
 
-static bool scratch_create(ScratchBlock &b, size_t bytes) {
-  // four sizes from one power of two to the next: calls of slightly different sizes share a block
+// four sizes from one power of two to the next: calls of slightly different sizes share a block
+size_t scratch_block_bytes(size_t bytes) {
   size_t step = size_t(16) << 20;
   while (8 * step < bytes) step *= 2;
-  const size_t up = (bytes + step - 1) / step * step;
+  return (bytes + step - 1) / step * step;
+}
+
+static bool scratch_create(ScratchBlock &b, size_t bytes) {
+  const size_t up = scratch_block_bytes(bytes);
   if (!device_room(up)) return false;
   if (cudaEventCreateWithFlags(&b.done, cudaEventDisableTiming) == cudaSuccess) {
     if (cudaMalloc(&b.p, up) == cudaSuccess) {

@@ -75,6 +75,8 @@ class ScratchLease {
   char *captured_ = nullptr;       // graph allocation
   ScratchBlock *block_ = nullptr;  // held, with its device's lock
 };
+// Size of a block for that many bytes.
+size_t scratch_block_bytes(size_t bytes);
 // Whether the device has twice these bytes free.
 bool device_room(size_t bytes);
 // Gives the kept blocks and the pool's unused memory back to the device.

@@ -16,13 +16,15 @@ overlaps with batches already on the device.
 
 Admission by device memory: at start the server measures the free device
 memory and keeps ``budget = free - reserve``.  Every slot owns a fixed device
-workspace of ``slot_bytes`` (by default twice the largest workspace of a
-batch at the server's limits, and at most budget / slots), allocated once, and
+workspace of ``slot_bytes``, allocated once, and
 runs its batches in it (``gm_batch_run_ws``): no batch takes an allocation
 from the library's stream-ordered pool, whose growth under load was measured
-to stall a launch for up to a second.  A batch is admitted only if its
-workspace (``gm_batch_workspace_bytes``) fits a slot; a single request that
-cannot fit even alone is rejected with an error.
+to stall a launch for up to a second.  By default that is, for a batch at the
+server's limits, its full workspace (``gm_batch_workspace_bytes``) and the
+least it needs (``gm_batch_workspace_min_bytes``) once more, as room for other
+mixes of sizes, and at most budget / slots.  A batch is admitted if the least
+it needs fits a slot; a single request that cannot fit even alone is rejected
+with an error.
 
 Latency of a request = completion time - submission time (host clock); the
 server records both for p50/p99.
@@ -85,9 +87,10 @@ class MsmServer:
         self.budget = mem_budget if mem_budget is not None else max(0, free - mem_reserve)
         self.slots = [_Slot(torch, self.dev, max_points, scalar_limbs, max_batch) for _ in range(slots)]
         if slot_bytes is None:
-            need = max((gm.batch_workspace_bytes(t, sz, scalar_limbs=scalar_limbs) for _, t, sz in self._limit_shapes()),
-                       default=0)
-            slot_bytes = min(self.budget // max(1, slots), 2 * need)
+            need = max((gm.batch_workspace_bytes(t, sz, scalar_limbs=scalar_limbs) +
+                        gm.batch_workspace_min_bytes(t, sz, scalar_limbs=scalar_limbs)
+                        for _, t, sz in self._limit_shapes()), default=0)
+            slot_bytes = min(self.budget // max(1, slots), need)
         self.slot_bytes = int(slot_bytes) // 256 * 256
         for sl in self.slots:
             sl.ws = torch.empty(max(256, self.slot_bytes), dtype=torch.uint8, device=self.dev)
@@ -155,7 +158,7 @@ class MsmServer:
     def _warmup(self):
         torch = self.torch
         for group, table, sizes in self._limit_shapes():
-            if gm.batch_workspace_bytes(table, sizes, scalar_limbs=self.limbs) > self.slot_bytes:
+            if gm.batch_workspace_min_bytes(table, sizes, scalar_limbs=self.limbs) > self.slot_bytes:
                 continue
             words = gm.G1P_WORDS if group == 1 else gm.G2P_WORDS
             total = int(sum(sizes))
@@ -200,7 +203,7 @@ class MsmServer:
             if len(take) == self.max_batch or points + n > self.max_points:
                 break
             trial = sizes + [n]
-            need = gm.batch_workspace_bytes(table, trial, scalar_limbs=self.limbs)
+            need = gm.batch_workspace_min_bytes(table, trial, scalar_limbs=self.limbs)
             if need > self.slot_bytes:
                 if not take:
                     # cannot fit even alone in a slot's workspace
@@ -217,7 +220,7 @@ class MsmServer:
             return None
         for r in take:
             self.pending.remove(r)
-        return group, take, gm.batch_workspace_bytes(table, sizes, scalar_limbs=self.limbs)
+        return group, take, gm.batch_workspace_min_bytes(table, sizes, scalar_limbs=self.limbs)
 
     def _launch(self, slot, group, reqs, nbytes):
         torch = self.torch

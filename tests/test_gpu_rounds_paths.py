@@ -49,3 +49,71 @@ def test_plan_modes_agree_word_for_word(cuda, tabled):
     assert torch.equal(queued, classes) and torch.equal(classes, again)
     plan.close()
     table.close()
+
+
+@pytest.mark.parametrize("group,tabled", [(1, False), (1, True), (2, False)])
+def test_batch_in_workspaces_of_either_size(cuda, group, tabled):
+    """In the reported size the batch runs as it does from the pool, word for
+    word and launch for launch; in the least accepted size without the rounds,
+    the same points; below that it is refused."""
+    table, sizes, wins, sc, want = make_batch(cuda, group=group, tabled=tabled)
+    least = gm.batch_workspace_min_bytes(table, sizes, window_bits=wins)
+    full = gm.batch_workspace_bytes(table, sizes, window_bits=wins)
+    assert full > least + (256 << 20)
+    gm.launch_count_reset()
+    pooled = gm.batch_run(table, sizes, sc, window_bits=wins)
+    n_pooled = gm.launch_count_reset()
+    guard = 1 << 20
+    ws = torch.zeros(full + guard, dtype=torch.uint8, device=cuda)
+    ws[full:] = 77
+    outs = {}
+    for name, size in (("full", full), ("least", least), ("short", full - (64 << 20))):
+        if name == "least":
+            ws[least:] = 77
+        outs[name] = gm.batch_run(table, sizes, sc, window_bits=wins, workspace=ws[:size])
+        outs[name + "_launches"] = gm.launch_count_reset()
+        if name != "short":
+            assert bool((ws[size:size + guard] == 77).all())
+    torch.cuda.synchronize()
+    assert torch.equal(outs["full"], pooled) and outs["full_launches"] == n_pooled
+    check(outs["least"], want, group)
+    assert outs["least_launches"] < n_pooled
+    check(outs["short"], want, group)
+    with pytest.raises(gm.MSMError):
+        gm.batch_run(table, sizes, sc, window_bits=wins, workspace=ws[:least - 1])
+    table.close()
+
+
+def test_reported_size_covers_the_pooled_run(cuda):
+    """gm_batch_run takes no more device memory than gm_batch_workspace_bytes reports."""
+    table, sizes, wins, sc, want = make_batch(cuda)
+    out = torch.empty((len(sizes), gm.G1P_WORDS), dtype=torch.int64, device=cuda)
+    gm.batch_run(table, sizes[:4], sc[:int(sizes[:4].sum())], window_bits=wins[:4], out=out[:4])
+    gm.trim_memory()
+    before = torch.cuda.mem_get_info()[0]
+    gm.batch_run(table, sizes, sc, window_bits=wins, out=out)
+    torch.cuda.synchronize()
+    taken = before - torch.cuda.mem_get_info()[0]
+    check(out, want)
+    full = gm.batch_workspace_bytes(table, sizes, window_bits=wins)
+    assert taken <= full + (128 << 20)  # the pool grows by whole chunks
+    table.close()
+
+
+def test_server_slots_hold_the_rounds(cuda):
+    """A server's full batch runs in its slot as it would from the pool."""
+    from gpu_msm_b200 import serving
+    table, sizes, wins, sc, want = make_batch(cuda)
+    server = serving.MsmServer({1: table}, max_batch=64, max_points=1 << 18, slots=2)
+    for _, t, sz in server._limit_shapes():
+        assert gm.batch_workspace_bytes(t, sz) <= server.slot_bytes
+    sz = [int(s) for s in sizes[:64]]
+    rows = int(sum(sz))
+    gm.launch_count_reset()
+    pooled = gm.batch_run(table, sz, sc[:rows])
+    n = gm.launch_count_reset()
+    own = gm.batch_run(table, sz, sc[:rows], workspace=server.slots[0].ws)
+    assert gm.launch_count_reset() == n
+    torch.cuda.synchronize()
+    assert torch.equal(own, pooled)
+    table.close()
