@@ -639,14 +639,11 @@ class ResidentBases:
 
     def windows_for(self, sizes, scalar_limbs: int = 5):
         """Per-MSM window widths to pass to a plan: 0 (the library picks the
-        cheapest fixed-base table) when the set has tables; one width for all
-        of a small batch; else the tuned widths."""
+        cheapest fixed-base table) when the set has tables, else
+        ``batch_widths``."""
         if self.precomputed:
             return [0] * len(sizes)
-        sizes = np.asarray(sizes, dtype=np.int64)
-        if len(sizes) > 1 and int(sizes.sum()) <= BATCH_ONE_CLASS:
-            return [batch_window(sizes, scalar_limbs)] * len(sizes)
-        return [tuned_window(self.group, int(s), scalar_limbs) for s in sizes]
+        return batch_widths(self.group, sizes, scalar_limbs)
 
     def msm(self, scalars, offset: int = 0, n: int = None, window_bits: int = 0, out=None, stream=None):
         """Asynchronous MSM over entries [offset, offset + n)."""
@@ -707,24 +704,41 @@ def tuned_params(group: int, n: int, scalar_limbs: int = 5):
     return default_window(group, n, scalar_limbs), 1, 4
 
 
-# Up to this many points in all, a batch takes one window width.  Every width
-# is a class with its own sort, fix-up and reduction, which a small batch does
-# not fill the GPU with.  B200, tuned widths per MSM -> one width: 20 G2 MSMs of
-# 2^6..2^12 points (25 k in all) 4.84 -> 3.60 ms, 20 such G1 MSMs 2.14 -> 1.50 ms,
-# 40 G1 MSMs of 2^10..2^14 (209 k) 5.43 -> 4.85 ms; 256 G2 MSMs of 2^8..2^12
-# (357 k) 26.6 -> 29.4 ms, so not there.
-BATCH_ONE_CLASS = 1 << 18
+# Up to this many points and MSMs, a batch may take one window width.  Every
+# width is a class with its own sort, fix-up and reduction, which a small batch
+# does not fill the GPU with.  Beyond, it does: 224 G1 MSMs of 2^7..2^10 points
+# 4.51 -> 4.02 ms on one width, 300 of 2^4..2^10 4.12 -> 4.53 ms (B200, plan runs).
+BATCH_ONE_POINTS, BATCH_ONE_MSMS = 1 << 18, 200
+# A (point, window) entry and a bucket, in products, and a further class of a
+# batch (0.25 ms): fits to 41 batches of 2 to 2000 MSMs at up to 10 widths each
+# (0.51 and 3.1 ns for G1, 1.3 and 9.7 ns for G2).
+BATCH_ENTRY, BATCH_BUCKET, BATCH_CLASS = 10, 60, 2e6
 
 
-def batch_window(sizes, scalar_limbs: int = 5) -> int:
-    """One window width for a small batch: 10 products per (point, window) and
-    38 per bucket, least over all its MSMs together."""
+def batch_widths(group: int, sizes, scalar_limbs: int = 5) -> list:
+    """Window width of every MSM of a batch without fixed-base tables: its
+    tuned one, or one width from among the tuned ones' range for all of a small
+    batch where that costs less than the classes of the tuned widths.
+
+    B200, tuned widths -> these: over 40 random small batches 0.84 of the time
+    as plans, 0.68 as transient batches.  20 MSMs of 2^6..2^12 points (15 k in
+    all) G1 1.85 -> 1.20 ms, G2 4.19 -> 2.75; 28 of 2^10..2^14 (144 k) G1 4.27 ->
+    3.69, G2 10.86 -> 9.08; 250000 points and 50 of 8 keep two widths."""
+    sizes = np.asarray(list(sizes), dtype=np.int64)
+    tuned = np.array([tuned_window(group, int(s), scalar_limbs) for s in sizes], dtype=np.int64)
+    widths = sorted(set(tuned.tolist()))
+    total, count = int(sizes.sum()), len(sizes)
+    if len(widths) < 2 or total > BATCH_ONE_POINTS or count > BATCH_ONE_MSMS:
+        return tuned.tolist()
     bits = min(64 * scalar_limbs, 299)
-    total, count = int(np.sum(sizes)), len(sizes)
 
-    def cost(c):
-        return 10 * total * (bits // c + 1) + 38 * count * (64 * scalar_limbs // c + 1) * 2 ** (c - 1)
-    return min(range(3, 13), key=cost)
+    def cost(points, msms, c):
+        return BATCH_ENTRY * points * (bits // c + 1) + BATCH_BUCKET * msms * (64 * scalar_limbs // c + 1) * 2 ** (c - 1)
+    classes = sum(cost(int(sizes[tuned == c].sum()), int((tuned == c).sum()), c) for c in widths)
+    one = min(range(widths[0], widths[-1] + 1), key=lambda c: cost(total, count, c))
+    if cost(total, count, one) < classes + BATCH_CLASS * (len(widths) - 1):
+        return [one] * count
+    return tuned.tolist()
 
 
 def tuned_window(group: int, n: int, scalar_limbs: int = 5) -> int:
