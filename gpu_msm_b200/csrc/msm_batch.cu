@@ -103,12 +103,16 @@ void plan_rounds(gm::BatchPlan &plan) {
 // A further class of a batch costs about TABLE_CLASS products' time whatever
 // its size (its own sort, fix-up and reduction launches, 0.2 ms), so all take
 // the table that is best for the whole batch unless the best one for each
-// saves more.  B200, each MSM's own best at 28 per bucket -> this rule: 40 MSMs
+// saves more, or the class would hold more entries than 32-bit offsets reach.
+// B200, each MSM's own best at 28 per bucket -> this rule: 40 MSMs
 // of 2^8..2^14 points over widths 11 and 14 3.10 -> 2.52 ms, 24 of 2^10..2^16
 // 5.67 -> 5.38 ms.
 constexpr double TABLE_CLASS = 4e6;
 std::vector<int> choose_tables(const gm_bases *b, int scalar_limbs, int count, const int64_t *sizes) {
   std::vector<int> each(count, 0);
+  auto cost = [&](int64_t n, int c) {
+    return 10.0 * (double)n * (64.0 * scalar_limbs / c) + 50.0 * (double)(1 << (c - 1));
+  };
   double best_all = 0, each_sum = 0;
   int c_all = 0;
   std::map<int, int> used;
@@ -116,9 +120,8 @@ std::vector<int> choose_tables(const gm_bases *b, int scalar_limbs, int count, c
     double best = 0;
     for (const auto &t : b->tables) {
       if (t.W < gm::windows_for(t.c, scalar_limbs)) continue;
-      const double cost = 10.0 * (double)sizes[i] * (64.0 * scalar_limbs / t.c) + 50.0 * (double)(1 << (t.c - 1));
-      if (each[i] == 0 || cost < best) {
-        best = cost;
+      if (each[i] == 0 || cost(sizes[i], t.c) < best) {
+        best = cost(sizes[i], t.c);
         each[i] = t.c;
       }
     }
@@ -128,15 +131,18 @@ std::vector<int> choose_tables(const gm_bases *b, int scalar_limbs, int count, c
   if (used.size() < 2) return each;
   for (const auto &t : b->tables) {
     if (t.W < gm::windows_for(t.c, scalar_limbs)) continue;
-    double cost = 0;
-    for (int i = 0; i < count; i++)
-      cost += 10.0 * (double)sizes[i] * (64.0 * scalar_limbs / t.c) + 50.0 * (double)(1 << (t.c - 1));
-    if (c_all == 0 || cost < best_all) {
-      best_all = cost;
+    double all = 0, entries = 0;
+    for (int i = 0; i < count; i++) {
+      all += cost(sizes[i], t.c);
+      entries += (double)sizes[i] * gm::windows_for(t.c, scalar_limbs);
+    }
+    if (entries < 4294967296.0 && (c_all == 0 || all < best_all)) {
+      best_all = all;
       c_all = t.c;
     }
   }
-  if (best_all <= each_sum + TABLE_CLASS * (double)(used.size() - 1)) each.assign(count, c_all);
+  if (c_all && best_all <= each_sum + TABLE_CLASS * (double)(used.size() - 1))
+    each.assign(count, c_all);
   return each;
 }
 

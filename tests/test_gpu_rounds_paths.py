@@ -117,3 +117,15 @@ def test_server_slots_hold_the_rounds(cuda):
     torch.cuda.synchronize()
     assert torch.equal(own, pooled)
     table.close()
+
+
+def test_tables_within_32_bit_offsets(cuda):
+    """Two widths whose one class would hold more than 2^32 entries stay two: the batch is planned, not refused."""
+    n = 1 << 12
+    logs = wl.make_base_logs(n, seed=3)
+    table = gm.ResidentBases(gm.generator_mul_batch(dev(logs, cuda)), group=1).precompute(4).precompute(16)
+    # all but the last take width 16, 4 entries short of 2^32; the last one width 4
+    sizes = np.array([n] * 49930 + [2991, 2991, 2990, 1], dtype=np.int64)
+    assert int(sizes[:-1].sum()) * 21 == 2 ** 32 - 4
+    assert gm.batch_workspace_min_bytes(table, sizes) > 0
+    table.close()
