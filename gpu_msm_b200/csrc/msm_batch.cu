@@ -98,7 +98,8 @@ void plan_rounds(gm::BatchPlan &plan) {
 }
 
 // Window widths of MSMs over fixed-base tables (0 without a table for the
-// scalars).  An MSM costs 10 products per (point, window) and, with its single
+// scalars, or where the caller gives a width).  An MSM costs 10 products per
+// (point, window) and, with its single
 // bucket set, 50 per bucket (two additions of 14 and the upper levels' share).
 // A further class of a batch costs about TABLE_CLASS products' time whatever
 // its size (its own sort, fix-up and reduction launches, 0.2 ms), so all take
@@ -108,8 +109,10 @@ void plan_rounds(gm::BatchPlan &plan) {
 // of 2^8..2^14 points over widths 11 and 14 3.10 -> 2.52 ms, 24 of 2^10..2^16
 // 5.67 -> 5.38 ms.
 constexpr double TABLE_CLASS = 4e6;
-std::vector<int> choose_tables(const gm_bases *b, int scalar_limbs, int count, const int64_t *sizes) {
+std::vector<int> choose_tables(const gm_bases *b, int scalar_limbs, int count, const int64_t *sizes,
+                               const int32_t *window_bits) {
   std::vector<int> each(count, 0);
+  auto free_width = [&](int i) { return !(window_bits && window_bits[i] > 0); };
   auto cost = [&](int64_t n, int c) {
     return 10.0 * (double)n * (64.0 * scalar_limbs / c) + 50.0 * (double)(1 << (c - 1));
   };
@@ -117,6 +120,7 @@ std::vector<int> choose_tables(const gm_bases *b, int scalar_limbs, int count, c
   int c_all = 0;
   std::map<int, int> used;
   for (int i = 0; i < count; i++) {
+    if (!free_width(i)) continue;
     double best = 0;
     for (const auto &t : b->tables) {
       if (t.W < gm::windows_for(t.c, scalar_limbs)) continue;
@@ -133,8 +137,9 @@ std::vector<int> choose_tables(const gm_bases *b, int scalar_limbs, int count, c
     if (t.W < gm::windows_for(t.c, scalar_limbs)) continue;
     double all = 0, entries = 0;
     for (int i = 0; i < count; i++) {
-      all += cost(sizes[i], t.c);
-      entries += (double)sizes[i] * gm::windows_for(t.c, scalar_limbs);
+      const bool here = free_width(i);
+      if (here) all += cost(sizes[i], t.c);
+      if (here || window_bits[i] == t.c) entries += (double)sizes[i] * gm::windows_for(t.c, scalar_limbs);
     }
     if (entries < 4294967296.0 && (c_all == 0 || all < best_all)) {
       best_all = all;
@@ -142,7 +147,8 @@ std::vector<int> choose_tables(const gm_bases *b, int scalar_limbs, int count, c
     }
   }
   if (c_all && best_all <= each_sum + TABLE_CLASS * (double)(used.size() - 1))
-    each.assign(count, c_all);
+    for (int i = 0; i < count; i++)
+      if (free_width(i)) each[i] = c_all;
   return each;
 }
 
@@ -159,7 +165,7 @@ int build_classes(const gm_bases *b, int scalar_limbs, int count, const int64_t 
   if (!b || count <= 0 || !sizes || scalar_limbs < 1 || scalar_limbs > gm::MAX_SCALAR_LIMBS) return gm::GM_ERR_ARG;
   int rc = gm::select_device((uint32_t)b->dev);
   if (rc) return rc;
-  const std::vector<int> table_c = choose_tables(b, scalar_limbs, count, sizes);
+  const std::vector<int> table_c = choose_tables(b, scalar_limbs, count, sizes, window_bits);
   std::map<int, std::vector<int>> by_c;
   std::vector<int64_t> sc_row(count + 1, 0);
   for (int i = 0; i < count; i++) {

@@ -129,3 +129,24 @@ def test_tables_within_32_bit_offsets(cuda):
     assert int(sizes[:-1].sum()) * 21 == 2 ** 32 - 4
     assert gm.batch_workspace_min_bytes(table, sizes) > 0
     table.close()
+
+
+def test_given_widths_do_not_sway_the_others(cuda):
+    """MSMs with a width of their own are left out of the choice of a table for the rest."""
+    n = 1 << 15
+    logs = wl.make_base_logs(n, seed=4)
+    table = gm.ResidentBases(gm.generator_mul_batch(dev(logs, cuda)), group=1).precompute(6).precompute(14)
+    small, large = [300] * 8 + [2000] * 2, [n] * 12
+    alone = gm.BatchPlan(table, small).classes()
+    sizes = small + large
+    wins = [0] * len(small) + [9] * len(large)
+    plan = gm.BatchPlan(table, sizes, window_bits=wins)
+    assert [c for c in plan.classes() if c[0] != 9] == alone
+    sc = wl.make_scalars(sum(sizes), seed=5)
+    out = plan.run(dev(sc, cuda))
+    torch.cuda.synchronize()
+    res = oracle.proj_to_affine(gm.to_numpy_proj(out))
+    for i, w in enumerate(wl.expected_logs(sizes, sc, logs)):
+        assert oracle.same_point(res[i:i + 1], oracle.generator_multiple(w)), i
+    plan.close()
+    table.close()
