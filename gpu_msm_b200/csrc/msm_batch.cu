@@ -107,8 +107,9 @@ void plan_rounds(gm::BatchPlan &plan) {
 // saves more, or the class would hold more entries than 32-bit offsets reach.
 // B200, each MSM's own best at 28 per bucket -> this rule: 40 MSMs
 // of 2^8..2^14 points over widths 11 and 14 3.10 -> 2.52 ms, 24 of 2^10..2^16
-// 5.67 -> 5.38 ms.
-constexpr double TABLE_CLASS = 4e6;
+// 5.67 -> 5.38 ms; 60 random batches 0.92 of the time (with 4e6 two of them 1.06
+// and 1.33 of it, a large MSM beside 30 tiny ones).
+constexpr double TABLE_CLASS = 2.5e6;
 std::vector<int> choose_tables(const gm_bases *b, int scalar_limbs, int count, const int64_t *sizes,
                                const int32_t *window_bits) {
   std::vector<int> each(count, 0);
