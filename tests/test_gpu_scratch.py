@@ -134,3 +134,30 @@ def test_without_room(case):
     assert oracle.same_point(same, oracle.proj_to_affine(gm.to_numpy_proj(want)))
     names, out = phases(pts, sc)
     assert "affine" in names and torch.equal(out, want)
+
+
+def test_plan_without_room(case):
+    """A plan takes the rounds' memory where the device has four times as much free, else runs without: the same points."""
+    pts, sc, _ = case
+    table = gm.ResidentBases(pts[:4096].contiguous(), group=1)
+    sizes = [2000 + i for i in range(60)]
+    wins = [9] * 50 + [6] * 10
+    rows = sum(sizes)
+    gm.trim_memory()
+    torch.cuda.empty_cache()
+    outs, counts, taken = [], [], []
+    for leave in (None, 2200 << 20):
+        fill = torch.empty(free() - leave, dtype=torch.uint8, device=pts.device) if leave else None
+        plan = gm.BatchPlan(table, sizes, window_bits=wins)
+        taken.append(plan.workspace_bytes)
+        gm.launch_count_reset()
+        outs.append(plan.run(sc[:rows]))
+        torch.cuda.synchronize()
+        counts.append(gm.launch_count_reset())
+        plan.close()
+        del fill
+        torch.cuda.empty_cache()
+    assert counts[1] < counts[0] and taken[1] < taken[0]
+    a, b = (oracle.proj_to_affine(gm.to_numpy_proj(o)) for o in outs)
+    assert oracle.same_point(a, b)
+    table.close()
