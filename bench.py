@@ -43,7 +43,7 @@ LOG2N = 20
 G2_LOG2N = 18
 # the timed plain-MSM steps run round-robin over this many streams: one MSM's
 # latency-bound tail (upper reduction levels, window combine) then
-# overlaps the next MSM's accumulation (G1 2^20: 16.6 -> 15.3 ms per MSM)
+# overlaps the next MSM's accumulation (G1 2^20: 10.8 -> 10.1 ms per MSM)
 PIPELINE_STREAMS = 3
 # CPU baseline sample: the first 2^16 points (about 1 s per pass on 16 host
 # cores); the repo arm reports the median of CPU_RUNS passes

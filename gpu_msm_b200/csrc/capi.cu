@@ -258,8 +258,9 @@ int host_msm(Prj *result, const Aff *points, const uint64_t *scalars, int limbs,
     proj_zero(result);
     return gm::GM_OK;
   }
-  // the scalars go first on s; the points follow on a second stream, so
-  // their copy overlaps the sort (which reads only the scalars)
+  // the scalars go first on s; the points follow on a second stream, so that
+  // from page-locked memory their copy overlaps the sort (which reads only the
+  // scalars); from pageable memory it is done before the sort is enqueued
   cudaStream_t s, s2;
   if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) return gm::GM_ERR_STREAM;
   if (cudaStreamCreateWithFlags(&s2, cudaStreamNonBlocking) != cudaSuccess) {

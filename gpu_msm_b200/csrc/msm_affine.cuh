@@ -25,7 +25,8 @@
 // offsets.  A round reads records by index (the first one through the sorted
 // entries, with their signs) and writes records; x = y = 0 is infinity.  Keys
 // (buckets) are processed in chunks of whole groups so that the two buffers
-// the rounds alternate between stay within AFF_SCRATCH bytes.
+// the rounds alternate between stay within AFF_SCRATCH bytes; a single group may
+// take twice that (MSMs of 2^25 points), and a larger one runs without rounds.
 #pragma once
 #include <algorithm>
 #include <vector>

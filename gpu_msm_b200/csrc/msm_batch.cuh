@@ -68,9 +68,9 @@ struct BatchPlan {
   // in one persistent launch over a device work queue (k_accumulate_queue)
   // between the classes' sorts and their fix-ups; false = one pipeline per
   // class on its own stream, every kernel of a class a full-GPU launch.
-  // The 512-MSM batch (2^8..2^16 points, 2^16-point table) measured 145.3 ms
-  // queued against 148.5-149.7 ms per class on B200, and 97.1 against
-  // 97.4 ms with fixed-base window tables.  Transient batches
+  // The 512-MSM batch (2^8..2^16 points, 2^16-point table) measured 97.7 ms
+  // queued against 99.2 ms per class on B200, and 67.0 against 67.5 ms with
+  // fixed-base window tables.  Transient batches
   // (gm_batch_run) run their classes in order on the caller's stream.
   bool queue = true;
   char *acc_desc = nullptr;      // AccClass<F>[classes] (owned)

@@ -154,7 +154,7 @@ static std::mutex g_pin_mu;
 static std::vector<void *> g_pin_free;
 // Slots whose last copy is still pending: returned to the free list once
 // their event has completed.  A host function per release would cost a
-// driver round trip (~0.2 ms of stream time on B200 boxes) for nothing.
+// driver round trip (~0.2 ms of stream time) for nothing.
 struct PendingSlot {
   void *slot;
   cudaEvent_t ev;

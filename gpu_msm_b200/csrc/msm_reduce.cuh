@@ -32,7 +32,7 @@ template <class F>
 constexpr int COMBINE_THREADS = 32 * (COMBINE_WARPS + Chain<F>::WARPS);
 constexpr int W_FILL = 16;        // warps per SM that keep its schedulers busy with dependent point operations
 constexpr int ACC_WARP_MIN = 4;    // entries of a slice on a warp, at least
-constexpr int ACC_WARP_MAX = 16;   // and at most; above W_SLICES slices of these, threads take the slices
+constexpr int ACC_WARP_MAX = 16;   // and at most; beyond four times W_FILL warps per SM of these, threads take the slices
 constexpr int ACC_THREAD_MIN = 16;  // entries of a slice on a thread, at least
 constexpr int RED_THREAD_MIN = 3;  // level 0 goes to threads above this many buckets per thread of a wave
 

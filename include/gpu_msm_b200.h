@@ -141,7 +141,8 @@ int gm_g2_msm_device_c(gm_stream_t stream, uint32_t gpu_index, G2ProjectivePoint
 /* MSM with an affine result (Montgomery form; infinity flag set for the
  * identity), the device form of point_msm_async<G1Point>/<G2Point>
  * (include/curve.h:238, src/curve.cu:2763), which returns an affine point.
- * Asynchronous; the conversion to affine runs on the device. */
+ * Asynchronous; the conversion to affine runs on the device.  n == 0 writes
+ * the point at infinity. */
 int gm_g1_msm_device_affine(gm_stream_t stream, uint32_t gpu_index, G1Point *d_result, const G1Point *d_points,
                             const uint64_t *d_scalars, int scalar_limbs, int n);
 int gm_g2_msm_device_affine(gm_stream_t stream, uint32_t gpu_index, G2Point *d_result, const G2Point *d_points,
@@ -234,8 +235,8 @@ int gm_batch_plan_create_tuned(const gm_bases *b, int scalar_limbs, int count, c
  * accumulation of every window class in one persistent launch over a device
  * work queue of (class, 32 slices) items, between the classes' sorts and
  * their fix-ups; 0 = one pipeline per window class, each on its own stream
- * with full-GPU kernels.  Results are identical; the mode only changes
- * scheduling. */
+ * with full-GPU kernels.  Results are identical, word for word; the mode only
+ * changes scheduling. */
 int gm_batch_plan_set_queue(gm_batch_plan *p, int on);
 int gm_batch_plan_destroy(gm_batch_plan *plan);
 int64_t gm_batch_plan_bytes(const gm_batch_plan *plan);
@@ -403,7 +404,8 @@ int gm_g1_sum_projective_host(G1ProjectivePoint *out, const G1ProjectivePoint *i
 
 /* Measurement hooks (no reference counterpart).
  * gm_profile_enable: while on, every MSM records CUDA events on its stream at
- *   its phase boundaries (pack, sort, accumulate, fixup, reduce, combine).
+ *   its phase boundaries (sort, pack, affine, accumulate, fixup, reduce, combine;
+ *   pack and affine where the call has them).
  * gm_profile_collect: waits for those events and returns up to `max`
  *   per-phase milliseconds in launch order, with their names comma-separated
  *   in `names`; clears the record.
