@@ -39,7 +39,8 @@ constexpr int AFF_THREADS = 128;
 constexpr int AFF_BATCH = 64;       // additions that share an inversion, at most
 constexpr int AFF_MIN = 16;         // outputs of a thread, at least (a shorter run spends more on its inversion)
 constexpr int AFF_MAX_ROUNDS = 8;
-// Outputs per thread of the last round, at least.  Measured with 10 / 16 / 24
+// Outputs per thread of the last round, at least, for both groups.  Flat from 10
+// to 16 for single MSMs; not measured below 10 or for batches.  With 10 / 16 / 24
 // / 40: G1 2^20 11.52 / 11.41 / 11.38 / 11.40 ms, G1 2^18 4.23 / 4.18 / 4.18 /
 // 4.25, G1 200000 3.41 / 3.34 / 3.46 / 3.46, G2 130000 6.18 / 6.13 / 6.48 / 6.47,
 // G2 65536 4.33 / 4.27 / 4.60 / 4.60 (without rounds: 13.66, 4.56, 3.77, 7.23, 4.60).
