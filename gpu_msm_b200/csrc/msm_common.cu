@@ -386,6 +386,7 @@ int trim_memory(int dev) {
   const int rc = device_state(dev, &st);
   if (rc) return rc;
   GM_CHECK(cudaMemPoolTrimTo(st->pool, 0));
+  GM_CHECK(cudaDeviceGraphMemTrim(dev));  // of captured calls whose graphs are gone
   return GM_OK;
 }
 

@@ -100,7 +100,8 @@ int g2_msm_limbs_wrapper(G2ProjectivePoint *result, const G2Point *points, const
  * device: the unused part of the stream-ordered pool that workspaces come
  * from, and the scratch blocks of large MSMs: one per call in flight (0.5 to
  * 3.5 GiB, 7 GiB after single MSMs of 2^25 points), at most four, which calls on
- * further streams take in turn.  Waits for the device.  Later calls take memory
+ * further streams take in turn; and the memory of graphs that have been
+ * destroyed.  Waits for the device.  Later calls take memory
  * again.  No reference counterpart (its callers own the scratch buffers). */
 int gm_trim_memory(uint32_t gpu_index);
 

@@ -161,3 +161,23 @@ def test_plan_without_room(case):
     a, b = (oracle.proj_to_affine(gm.to_numpy_proj(o)) for o in outs)
     assert oracle.same_point(a, b)
     table.close()
+
+
+def test_graph_memory_is_given_back(case):
+    """A captured call's scratch is the graph's; destroyed and trimmed, the device has it again."""
+    pts, sc, want = case
+    out = torch.empty_like(want)
+    gm.trim_memory()
+    start = free()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, capture_error_mode="thread_local"):
+        gm.msm_device(pts, sc, window_bits=C, out=out)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, want)
+    held = start - free()
+    assert held > 256 << 20
+    g.reset()
+    del g
+    gm.trim_memory()
+    assert start - free() < held / 4
